@@ -1,27 +1,30 @@
-// Kernels of the sTDDFT ("std") density-fitting tensors (std/intor.f90):
-//  * k_std_df1c       (mu mu|P) for every orbital function mu: the diagonal of
-//                     the (aa|c) blocks, screened by Q_aa * Q_c
-//                     (intor_df1c, std/intor.f90:66-111);
-//  * k_std_df2c_half  the first half-transformation of intor_df2c_mo
-//                     (std/intor.f90:207-261) with the reference's two value
-//                     skips, summed over the partner shell a for every target
-//                     shell b and auxiliary shell c; the second half
-//                     (std/intor.f90:263-279) is then one GEMM per batch of
-//                     auxiliary functions, followed by k_std_pack;
+// Kernels of the sTDDFT ("std") density-fitting tensors (std/intor.f90). The
+// explicit blocks (ab|c) come from the class kernels of k_std3c_impl.cuh; here:
+//  * k_std_pair_size, k_std_pair_row, k_std_columns  the layout of the block
+//                     matrix: rows are the function pairs of the shell pairs
+//                     that meet the largest auxiliary Schwarz value, columns
+//                     the auxiliary functions in sorted class order;
+//  * k_std_half       the first half-transformation of intor_df2c_mo
+//                     (std/intor.f90:207-261) with the reference's skip of
+//                     half-transformed values (:269), summed over the partner
+//                     shell a for every target function nu; the second half
+//                     (:263-279) is then one GEMM per batch of auxiliary
+//                     functions, followed by k_std_pack;
+//  * k_std_block_norm ||(ab|c)|| of single blocks (the estimator study);
 //  * k_transpose      column-major transposition of the L^-1-applied results.
 //
-// Both integral kernels evaluate explicit spherical (ab|c) blocks, because the
-// reference drops individual integrals |(ab|c)| <= 1e-10 (REAL(4) literal) and
-// individual half-transformed values <= 1e-10 before summing; at the 8-atom
+// The reference drops individual integrals |(ab|c)| <= 1e-10 (REAL(4) literal)
+// and individual half-transformed values <= 1e-10 before summing; at the 8-atom
 // workload these skips move intor_df2c_mo by ~4e-9, so they are reproduced
-// triple by triple. A block of (ab|c) is built by McMurchie-Davidson like the
-// other kernels of the library:
-//   (ab|c)[(ma,mb)][m] = sum_(units u of ab) sum_(prims of c) sum_tuv
-//                        E_sph,u[(ma,mb)][tuv] X_(u,c)[tuv][m]
-// with X = pref sum_tau S_lc,m[tau] R_(tuv+tau)(alpha, P_u - C).
+// triple by triple, which is why the blocks are stored and not contracted on
+// the way.
 #include "boys.cuh"
 #include "k_std.cuh"
+#include "k_std3c.cuh"
 #include "md.cuh"
+
+#include <algorithm>
+#include <mutex>
 
 namespace pa {
 
@@ -32,18 +35,13 @@ struct BlockSync {
 };
 
 constexpr int kStdThreads = 128;
-// k_std_df2c_half: two blocks per SM (its shared memory: the integral
-// scratch and the half-transformed accumulator), so eight warps each
-constexpr int kStdHalfThreads = 256;
 constexpr int kLtot = 2 * PA_LMAX + PA_LAUXMAX;           // highest la + lb + lc
 constexpr int kNR = ncum(kLtot);                           // R entries of one build
 constexpr int kNHMax = ncum(2 * PA_LMAX);                  // Hermite components of a bra
 constexpr int kNCMax = 2 * PA_LAUXMAX + 1;                 // spherical aux functions
 constexpr int kNSMax = 2 * PA_LMAX + 1;                    // spherical orbital functions
 constexpr int kNabMax = kNSMax * kNSMax;
-constexpr int kMoChunk = 64;                               // MOs per df2c block
-constexpr double kSkip1 = static_cast<double>(1e-10f);     // std/intor.f90:247 (REAL(4))
-constexpr double kSkip2 = 1e-10;                           // std/intor.f90:269
+constexpr double kSkipHalf = 1e-10;                        // std/intor.f90:269
 
 // Shared scratch of block_3c.
 struct Blk3cScratch {
@@ -128,22 +126,6 @@ __device__ void block_3c(const StdArgs& a, int pair, int c, Blk3cScratch s) {
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kStdThreads) k_std_df1c(StdArgs a, double* __restrict__ Tt,
-                                                          int naux) {
-  __shared__ double scratch[kBlk3cDoubles];
-  const int c = blockIdx.x, sh = blockIdx.y;
-  const int pair = sh * (sh + 1) / 2 + sh;
-  if (a.Qab[pair] * a.Qc[c] < a.thresh) return;  // schwarz_estimate(a, a, c) < 1e-10
-  Blk3cScratch s = blk3c_scratch(scratch);
-  block_3c(a, pair, c, s);
-  const int4 sa = a.B.shell[sh], sc = a.X.shell[c];
-  const int na = 2 * sa.x + 1, NC = 2 * sc.x + 1;
-  for (int idx = threadIdx.x; idx < na * NC; idx += blockDim.x) {
-    const int i = idx / NC, m = idx - i * NC;
-    Tt[(sc.w + m) + static_cast<long long>(naux) * (sa.w + i)] = s.I[(i * na + i) * NC + m];
-  }
-}
-
 // ||(ab|c)||_2 of the block of pair rec_pair[blockIdx.y] and auxiliary shell
 // blockIdx.x (the estimator study of intor/benchmark.f90:96-118).
 __global__ void __launch_bounds__(kStdThreads) k_std_block_norm(StdArgs a, const int* __restrict__ rec_pair,
@@ -168,85 +150,234 @@ __global__ void __launch_bounds__(kStdThreads) k_std_block_norm(StdArgs a, const
   }
 }
 
-// One block per (aux shell c, target shell b, chunk of MOs).
-__global__ void __launch_bounds__(kStdHalfThreads) k_std_df2c_half(StdArgs a, int c0, int k0, int nmos,
-                                                               const double* __restrict__ mo,
-                                                               double* __restrict__ W, int moc) {
-  extern __shared__ double sm[];
-  Blk3cScratch s = blk3c_scratch(sm);
-  double* Cs = sm + kBlk3cDoubles;     // [kNSMax][moc]
-  double* Wacc = Cs + kNSMax * moc;    // [moc][nb][NC]
-  const int c = c0 + blockIdx.x, b = blockIdx.y;
-  const int mo0 = blockIdx.z * moc, nm = min(moc, nmos - mo0);
-  const int tid = threadIdx.x;
-  const int nbf = a.B.nsph;
-  const int4 sb = a.B.shell[b], sc = a.X.shell[c];
-  const int nb = 2 * sb.x + 1, NC = 2 * sc.x + 1;
-  const int nw = nm * nb * NC;
-  for (int i = tid; i < nw; i += blockDim.x) Wacc[i] = 0.0;
-  const double qc = a.Qc[c];
-  // partners in ascending order (the reference's loop order), tested
-  // kStdHalfThreads at a time: each thread tests one partner, the warps'
-  // ballots go to shared memory, and the block walks the surviving partners
-  // of the chunk bit by bit (warp by warp)
-  __shared__ unsigned s_alive[kStdHalfThreads / 32];
-  for (int sh0 = 0; sh0 < a.B.nshells; sh0 += kStdHalfThreads) {
-    {
-      const int sh = sh0 + tid;
-      bool alive = false;
-      if (sh < a.B.nshells) {
-        const int hi = max(sh, b), lo = min(sh, b);
-        alive = !(a.Qab[hi * (hi + 1) / 2 + lo] * qc < a.thresh);  // schwarz_estimate(a, b, c) >= 1e-10
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, alive);
-      if ((tid & 31) == 0) s_alive[tid >> 5] = m;
-    }
-    __syncthreads();
-    for (int wi = 0; wi < kStdHalfThreads / 32; ++wi) {
-      unsigned m = s_alive[wi];
-      while (m) {
-        const int sh = sh0 + 32 * wi + __ffs(m) - 1;
-        m &= m - 1;
-        const int hi = max(sh, b), lo = min(sh, b);
-        const int pair = hi * (hi + 1) / 2 + lo;
-        block_3c(a, pair, c, s);
-        const int4 sa = a.B.shell[sh];
-        const int na = 2 * sa.x + 1;
-        for (int i = tid; i < na * nm; i += blockDim.x) {
-          const int ii = i / nm, mm = i - ii * nm;
-          Cs[ii * moc + mm] = mo[(sa.w + ii) + static_cast<long long>(nbf) * (mo0 + mm)];
-        }
-        for (int i = tid; i < na * nb * NC; i += blockDim.x)
-          if (fabs(s.I[i]) <= kSkip1) s.I[i] = 0.0;
-        __syncthreads();
-        // h[mo][j][m] = sum_(i in a) C[i, mo] (a_i b_j | c_m); the stored block is
-        // (hi lo | c), so (a b|c) is its transpose when a < b
-        const bool a_first = sh >= b;
-        for (int idx = tid; idx < nw; idx += blockDim.x) {
-          const int mm = idx / (nb * NC), rem = idx - mm * (nb * NC);
-          const int j = rem / NC, m = rem - j * NC;
-          double h = 0.0;
-          for (int i = 0; i < na; ++i) {
-            const double iv = a_first ? s.I[(i * nb + j) * NC + m] : s.I[(j * na + i) * NC + m];
-            h = fma(Cs[i * moc + mm], iv, h);
-          }
-          if (fabs(h) > kSkip2) Wacc[idx] += h;
-        }
-      }
-    }
-    __syncthreads();  // s_alive is rewritten by the next chunk
+// keys[i] = Schwarz value of the i-th pair of the class-ordered list.
+__global__ void k_std_pair_keys(int n, const int* __restrict__ class_pair, const double* __restrict__ Qab,
+                                double* keys, int* vals) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  keys[i] = Qab[class_pair[i]];
+  vals[i] = i;
+}
+
+// Rows of the sorted pair i in the block matrix: all of its function pairs when
+// it meets the largest auxiliary Schwarz value, else none. The sorted values
+// fall within a class, so its surviving pairs are a prefix: nclass[c].
+__global__ void k_std_pair_size(StdArgs a, int n, const double* __restrict__ Q, const int* __restrict__ pair,
+                                const int* __restrict__ off, int nseg, const double* __restrict__ qmax, int* size,
+                                int* nclass) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double qm = *qmax;
+  const int2 ab = a.pair_ab[pair[i]];
+  const bool alive = !(Q[i] * qm < a.thresh);
+  size[i] = alive ? (2 * a.B.shell[ab.x].x + 1) * (2 * a.B.shell[ab.y].x + 1) : 0;
+  int c = 0;
+  while (c + 1 < nseg && i >= off[c + 1]) ++c;
+  if (alive && (i + 1 == off[c + 1] || Q[i + 1] * qm < a.thresh)) nclass[c] = i + 1 - off[c];
+}
+
+// First row per pair id (-1: no rows); the number of rows goes to *total.
+__global__ void k_std_pair_row(int n, const int* __restrict__ pair, const int* __restrict__ size,
+                               const int* __restrict__ first, int* row0, int* total) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  row0[pair[i]] = size[i] > 0 ? first[i] : -1;
+  if (i == n - 1) *total = first[i] + size[i];
+}
+
+// Columns: function m of sorted auxiliary shell i of class L is column
+// (functions of lower classes) + (i - off[L]) (2L + 1) + m.
+__global__ void k_std_columns(int n, const int* __restrict__ sorted, const double* __restrict__ Q,
+                              const int* __restrict__ off, int nseg, const int4* __restrict__ shell, int* col_fn,
+                              double* col_Q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int L = 0, base = 0;
+  while (L + 1 < nseg && i >= off[L + 1]) {
+    base += (off[L + 1] - off[L]) * (2 * L + 1);
+    ++L;
   }
-  __syncthreads();
-  for (int idx = tid; idx < nw; idx += blockDim.x) {
-    const int mm = idx / (nb * NC), rem = idx - mm * (nb * NC);
-    const int j = rem / NC, m = rem - j * NC;
-    const long long k = sc.w + m - k0;
-    W[(k * nmos + mo0 + mm) * nbf + sb.w + j] = Wacc[idx];
+  base += (i - off[L]) * (2 * L + 1);
+  for (int m = 0; m < 2 * L + 1; ++m) {
+    col_fn[base + m] = shell[sorted[i]].w + m;
+    col_Q[base + m] = Q[i];
   }
 }
 
-__global__ void k_std_pack(const double* __restrict__ Res, int nk, int nmos, int k0, int naux,
-                           double* __restrict__ Raw) {
+// Shell of every orbital function.
+__global__ void k_std_fn_shell(int n, const int4* __restrict__ shell, int* fn_shell) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  for (int m = 0; m < 2 * shell[i].x + 1; ++m) fn_shell[shell[i].w + m] = i;
+}
+
+// Ct[i * pld + p] = C[i, p], zero for p >= nmos.
+__global__ void k_std_mo_rows(const double* __restrict__ mo, int nbf, int nmos, int pld, double* __restrict__ Ct) {
+  const long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  if (idx >= static_cast<long long>(nbf) * pld) return;
+  const int i = static_cast<int>(idx / pld), p = static_cast<int>(idx - static_cast<long long>(i) * pld);
+  Ct[idx] = p < nmos ? mo[i + static_cast<long long>(nbf) * p] : 0.0;
+}
+
+// W[nu][p][k] = sum_a skip(sum_(i in a) C[i, p] (i nu|k)), partner shells a in
+// ascending order (the reference's), skip(h) = h where |h| > 1e-10, else 0.
+//
+// A block owns one target function nu, 64 columns k and 16 PT orbitals p; a
+// thread a PT x 4 tile of them, its partial sum over the functions of the
+// current shell beside its accumulator. The functions of the surviving partner
+// shells form one list of rows (a shell survives when its pair has rows and
+// meets the tile's largest auxiliary Schwarz value); 16 rows of (i nu|k) and of
+// C are staged at a time through three cp.async buffers, so a shell may
+// straddle two stages. Bound: the FP64 pipe, (functions + 2 per shell)
+// operations per (nu, k, p) and partner shell; no tensor cores, because the
+// skip needs every shell's sum on its own, and padding shells of 1, 3, 5, 7
+// functions to the depth of an FP64 mma (4) would cost 1.7 times the products.
+constexpr int kHalfCols = 64, kHalfRows = 16, kHalfStages = 3;
+constexpr int kHalfThreads = 256;
+constexpr int kHalfList = kHalfThreads * kNSMax;  // rows of one group of partner shells
+
+constexpr size_t half_smem(int pt) {
+  return sizeof(double) * kHalfStages * kHalfRows * (kHalfCols + 16 * pt) + sizeof(int) * 2 * kHalfList;
+}
+
+__device__ __forceinline__ void half_cp16(double* dst, const double* src) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src));
+}
+
+template <int PT>
+__global__ void __launch_bounds__(kHalfThreads, 2) k_std_half(StdHalfArgs h) {
+  constexpr int P = 16 * PT;
+  extern __shared__ __align__(16) double sm[];
+  double* Is = sm;                                             // [stage][row][kHalfCols]
+  double* Cs = Is + kHalfStages * kHalfRows * kHalfCols;       // [stage][row][P]
+  int* s_row = reinterpret_cast<int*>(Cs + kHalfStages * kHalfRows * P);  // row of the block matrix
+  int* s_fn = s_row + kHalfList;                               // partner function * 2 + (last of its shell)
+  __shared__ int s_cnt[kHalfThreads / 32];
+  __shared__ double s_q[kHalfThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nkt = (h.nk + kHalfCols - 1) / kHalfCols;
+  const int nu = blockIdx.x / nkt, k0 = (blockIdx.x - nu * nkt) * kHalfCols;
+  const int p0 = blockIdx.y * P;
+  const int b = h.fn_shell[nu];
+  const int4 sb = h.B.shell[b];
+  const int nb = 2 * sb.x + 1, j = nu - sb.w;
+  const int ncol2 = min(kHalfCols, h.ld - k0) / 2;  // 16-byte pieces of the tile's rows (ld is even)
+
+  double qmax = tid < kHalfCols && k0 + tid < h.nk ? h.col_Q[k0 + tid] : 0.0;
+  for (int o = 16; o > 0; o >>= 1) qmax = fmax(qmax, __shfl_xor_sync(0xffffffffu, qmax, o));
+  if (lane == 0) s_q[warp] = qmax;
+  __syncthreads();
+  qmax = fmax(s_q[0], s_q[1]);
+
+  const int kt = tid & 15, pt = tid >> 4;
+  double acc[PT][4], hh[PT][4];
+#pragma unroll
+  for (int q = 0; q < PT; ++q)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[q][i] = hh[q][i] = 0.0;
+
+  for (int sh0 = 0; sh0 < h.B.nshells; sh0 += kHalfThreads) {
+    // rows of this group's surviving partner shells, in shell order
+    const int sh = sh0 + tid;
+    int na = 0, r0 = -1, fn0 = 0;
+    if (sh < h.B.nshells) {
+      const int hi = max(sh, b), lo = min(sh, b);
+      const long long pair = static_cast<long long>(hi) * (hi + 1) / 2 + lo;
+      r0 = h.row0[pair];
+      if (r0 >= 0 && !(h.Qab[pair] * qmax < h.thresh)) {
+        const int4 sa = h.B.shell[sh];
+        na = 2 * sa.x + 1;
+        fn0 = sa.w;
+      }
+    }
+    int incl = na;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_cnt[warp] = incl;
+    __syncthreads();
+    int off = incl - na, total = 0;
+    for (int w = 0; w < kHalfThreads / 32; ++w) {
+      if (w < warp) off += s_cnt[w];
+      total += s_cnt[w];
+    }
+    for (int i = 0; i < na; ++i) {
+      s_row[off + i] = r0 + (sh >= b ? i * nb + j : j * na + i);
+      s_fn[off + i] = 2 * (fn0 + i) + (i == na - 1 ? 1 : 0);
+    }
+    __syncthreads();
+    const int nch = (total + kHalfRows - 1) / kHalfRows;
+    auto issue = [&](int c) {
+      if (c < nch) {
+        double* is = Is + (c % kHalfStages) * kHalfRows * kHalfCols;
+        double* cs = Cs + (c % kHalfStages) * kHalfRows * P;
+        const int nr = min(kHalfRows, total - c * kHalfRows);
+        for (int e = tid; e < kHalfRows * (kHalfCols / 2); e += kHalfThreads) {
+          const int r = e / (kHalfCols / 2), x = e % (kHalfCols / 2);
+          if (r < nr && x < ncol2)
+            half_cp16(is + r * kHalfCols + 2 * x,
+                      h.I + static_cast<long long>(s_row[c * kHalfRows + r]) * h.ld + k0 + 2 * x);
+        }
+        for (int e = tid; e < kHalfRows * (P / 2); e += kHalfThreads) {
+          const int r = e / (P / 2), x = e % (P / 2);
+          if (r < nr)
+            half_cp16(cs + r * P + 2 * x,
+                      h.Ct + static_cast<long long>(s_fn[c * kHalfRows + r] >> 1) * h.pld + p0 + 2 * x);
+        }
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+    };
+    issue(0);
+    issue(1);
+    for (int c = 0; c < nch; ++c) {
+      asm volatile("cp.async.wait_group 1;\n" ::);
+      __syncthreads();  // stage c has arrived; stage c - 1 is consumed
+      issue(c + 2);
+      const double* is = Is + (c % kHalfStages) * kHalfRows * kHalfCols + 2 * kt;
+      const double* cs = Cs + (c % kHalfStages) * kHalfRows * P + pt * PT;
+      const int nr = min(kHalfRows, total - c * kHalfRows);
+#pragma unroll 2
+      for (int r = 0; r < nr; ++r) {
+        const double2 x0 = *reinterpret_cast<const double2*>(is + r * kHalfCols);
+        const double2 x1 = *reinterpret_cast<const double2*>(is + r * kHalfCols + kHalfCols / 2);
+#pragma unroll
+        for (int q = 0; q < PT; ++q) {
+          const double cv = cs[r * P + q];
+          hh[q][0] = fma(cv, x0.x, hh[q][0]);
+          hh[q][1] = fma(cv, x0.y, hh[q][1]);
+          hh[q][2] = fma(cv, x1.x, hh[q][2]);
+          hh[q][3] = fma(cv, x1.y, hh[q][3]);
+        }
+        if (s_fn[c * kHalfRows + r] & 1)
+#pragma unroll
+          for (int q = 0; q < PT; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (fabs(hh[q][i]) > kSkipHalf) acc[q][i] += hh[q][i];
+              hh[q][i] = 0.0;
+            }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();  // the lists and stages are rewritten by the next group
+  }
+#pragma unroll
+  for (int q = 0; q < PT; ++q) {
+    const int p = p0 + pt * PT + q;
+    if (p >= h.nmos) continue;
+    double* w = h.W + (static_cast<long long>(nu) * h.nmos + p) * h.ld + k0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = i * (kHalfCols / 2) + 2 * kt;
+      if (c / 2 < ncol2) *reinterpret_cast<double2*>(w + c) = make_double2(acc[q][2 * i], acc[q][2 * i + 1]);
+    }
+  }
+}
+
+__global__ void k_std_pack(const double* __restrict__ Res, int nk, int ld, int nmos, const int* __restrict__ col_fn,
+                           int naux, double* __restrict__ Raw) {
   const long long npack = static_cast<long long>(nmos) * (nmos + 1) / 2;
   const long long total = npack * nk;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -257,8 +388,8 @@ __global__ void k_std_pack(const double* __restrict__ Res, int nk, int nmos, int
     while (static_cast<long long>(p) * (p + 1) / 2 > pk) --p;
     while (static_cast<long long>(p + 1) * (p + 2) / 2 <= pk) ++p;
     const int q = static_cast<int>(pk - static_cast<long long>(p) * (p + 1) / 2);
-    Raw[(k0 + kk) + static_cast<long long>(naux) * pk] =
-        Res[(static_cast<long long>(kk) * nmos + p) + static_cast<long long>(nk) * nmos * q];
+    Raw[col_fn[kk] + static_cast<long long>(naux) * pk] =
+        Res[kk + static_cast<long long>(ld) * (p + static_cast<long long>(nmos) * q)];
   }
 }
 
@@ -280,22 +411,97 @@ __global__ void k_transpose(const double* __restrict__ in, int rows, int cols, d
 
 }  // namespace
 
-int launch_std_df1c(const StdArgs& a, double* Tt, cudaStream_t s) {
-  if (a.B.nshells == 0 || a.X.nshells == 0) return 0;
-  dim3 grid(a.X.nshells, a.B.nshells);
-  k_std_df1c<<<grid, kStdThreads, 0, s>>>(a, Tt, a.X.nsph);
+namespace {
+
+const Std3cRow* std3c_rows() {
+  static Std3cRow table[2 * PA_LMAX + 1];
+  static std::once_flag once;
+  std::call_once(once, [] {
+    std3c_row_0(&table[0]);
+    std3c_row_1(&table[1]);
+    std3c_row_2(&table[2]);
+    std3c_row_3(&table[3]);
+    std3c_row_4(&table[4]);
+    std3c_row_5(&table[5]);
+    std3c_row_6(&table[6]);
+    std3c_row_7(&table[7]);
+    std3c_row_8(&table[8]);
+  });
+  return table;
+}
+
+template <int PT>
+int launch_half(const StdHalfArgs& h, cudaStream_t s) {
+  const size_t smem = half_smem(PT);
+  cudaFuncSetAttribute(k_std_half<PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const long long tiles = static_cast<long long>((h.nk + kHalfCols - 1) / kHalfCols) * h.B.nsph;
+  k_std_half<PT><<<dim3(static_cast<unsigned>(tiles), (h.nmos + 16 * PT - 1) / (16 * PT)), kHalfThreads, smem, s>>>(h);
   return 1;
 }
 
-int launch_std_df2c_half(const StdArgs& a, int c0, int c1, int k0, int nmos, const double* mo,
-                         double* W, cudaStream_t s) {
-  if (c1 <= c0 || a.B.nshells == 0 || nmos == 0) return 0;
-  const int moc = nmos < kMoChunk ? nmos : kMoChunk;
-  const size_t smem = sizeof(double) * (kBlk3cDoubles + kNSMax * moc + static_cast<size_t>(moc) * kNSMax * kNCMax);
-  cudaFuncSetAttribute(k_std_df2c_half, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  dim3 grid(c1 - c0, a.B.nshells, (nmos + moc - 1) / moc);
-  k_std_df2c_half<<<grid, kStdHalfThreads, smem, s>>>(a, c0, k0, nmos, mo, W, moc);
+}  // namespace
+
+int launch_std3c_class(int lab, int lc, const Std3cArgs& a, cudaStream_t s) {
+  return std3c_rows()[lab].launch[lc](a, s);
+}
+
+cudaError_t upload_std3c_rownorm(const double* rownorm, cudaStream_t s) {
+  for (int lab = 0; lab <= 2 * PA_LMAX; ++lab) {
+    const cudaError_t e = std3c_rows()[lab].upload_rownorm(rownorm, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+int launch_std_pair_keys(int n, const int* class_pair, const double* Qab, double* keys, int* vals, cudaStream_t s) {
+  if (n <= 0) return 0;
+  k_std_pair_keys<<<(n + 255) / 256, 256, 0, s>>>(n, class_pair, Qab, keys, vals);
   return 1;
+}
+
+int launch_std_pair_size(const StdArgs& a, int n, const double* Q, const int* pair, const int* off, int nseg,
+                         const double* qmax, int* size, int* nclass, cudaStream_t s) {
+  if (n <= 0) return 0;
+  k_std_pair_size<<<(n + 255) / 256, 256, 0, s>>>(a, n, Q, pair, off, nseg, qmax, size, nclass);
+  return 1;
+}
+
+int launch_std_pair_row(int n, const int* pair, const int* size, const int* first, int* row0, int* total,
+                        cudaStream_t s) {
+  if (n <= 0) return 0;
+  k_std_pair_row<<<(n + 255) / 256, 256, 0, s>>>(n, pair, size, first, row0, total);
+  return 1;
+}
+
+int launch_std_columns(int n, const int* sorted, const double* Q, const int* off, int nseg, const int4* shell,
+                       int* col_fn, double* col_Q, cudaStream_t s) {
+  if (n <= 0) return 0;
+  k_std_columns<<<(n + 255) / 256, 256, 0, s>>>(n, sorted, Q, off, nseg, shell, col_fn, col_Q);
+  return 1;
+}
+
+int launch_std_orbitals(const DevBasis& B, const double* mo, int nmos, int pld, int* fn_shell, double* Ct,
+                        cudaStream_t s) {
+  if (B.nshells <= 0 || nmos <= 0) return 0;
+  k_std_fn_shell<<<(B.nshells + 255) / 256, 256, 0, s>>>(B.nshells, B.shell, fn_shell);
+  const long long n = static_cast<long long>(B.nsph) * pld;
+  k_std_mo_rows<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(mo, B.nsph, nmos, pld, Ct);
+  return 2;
+}
+
+// Orbitals per thread: the fewest that cover nmos with one block column, at
+// most 4 (64 orbitals per block; PT = 4 keeps tile, sums and operands within
+// the 128 registers of two blocks per SM).
+int std_half_pt(int nmos) { return std::min(4, std::max(1, (nmos + 15) / 16)); }
+
+int launch_std_half(const StdHalfArgs& h, cudaStream_t s) {
+  if (h.nk <= 0 || h.B.nsph <= 0 || h.nmos <= 0) return 0;
+  switch (std_half_pt(h.nmos)) {
+    case 1: return launch_half<1>(h, s);
+    case 2: return launch_half<2>(h, s);
+    case 3: return launch_half<3>(h, s);
+    default: return launch_half<4>(h, s);
+  }
 }
 
 int launch_std_block_norms(const StdArgs& a, const int* rec_pair, int npairs, double* out, cudaStream_t s) {
@@ -310,11 +516,12 @@ int launch_std_block_norms(const StdArgs& a, const int* rec_pair, int npairs, do
   return done;
 }
 
-int launch_std_pack(const double* Res, int nk, int nmos, int k0, int naux, double* Raw, cudaStream_t s) {
+int launch_std_pack(const double* Res, int nk, int ld, int nmos, const int* col_fn, int naux, double* Raw,
+                    cudaStream_t s) {
   const long long total = static_cast<long long>(nmos) * (nmos + 1) / 2 * nk;
   if (total == 0) return 0;
   const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148 * 16));
-  k_std_pack<<<blocks, 256, 0, s>>>(Res, nk, nmos, k0, naux, Raw);
+  k_std_pack<<<blocks, 256, 0, s>>>(Res, nk, ld, nmos, col_fn, naux, Raw);
   return 1;
 }
 

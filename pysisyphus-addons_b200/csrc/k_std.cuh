@@ -20,19 +20,42 @@ struct StdArgs {
   const double* Qc = nullptr;        // aux shell -> Schwarz value
 };
 
-// Tt[P + naux * mu] = (mu mu|P) for surviving (a, a, c); other entries untouched
-// (std/intor.f90:66-111).
-int launch_std_df1c(const StdArgs& a, double* Tt, cudaStream_t s);
+// Layout of the block matrix (k_std.cu): Schwarz values of the class-ordered
+// pairs, rows of the sorted pairs and their number, columns of the sorted
+// auxiliary shells.
+int launch_std_pair_keys(int n, const int* class_pair, const double* Qab, double* keys, int* vals, cudaStream_t s);
+int launch_std_pair_size(const StdArgs& a, int n, const double* Q, const int* pair, const int* off, int nseg,
+                         const double* qmax, int* size, int* nclass, cudaStream_t s);
+int launch_std_pair_row(int n, const int* pair, const int* size, const int* first, int* row0, int* total,
+                        cudaStream_t s);
+int launch_std_columns(int n, const int* sorted, const double* Q, const int* off, int nseg, const int4* shell,
+                       int* col_fn, double* col_Q, cudaStream_t s);
 
-// Half-transformed, value-screened blocks of intor_df2c_mo (std/intor.f90:207-261)
-// for the auxiliary shells [c0, c1): W[((k - k0) * nmos + p) * nbf + nu] =
-// sum_a skip2(sum_(i in a) C[i, p] skip1((a b|k))) for nu in shell b, k in
-// [k0, k1) the functions of the shells. mo is C (nbf x nmos, column-major).
-int launch_std_df2c_half(const StdArgs& a, int c0, int c1, int k0, int nmos, const double* mo,
-                         double* W, cudaStream_t s);
+// fn_shell[nu] = shell of orbital function nu; Ct[nu * pld + p] = C[nu, p]
+// (zero for nmos <= p < pld). mo is C (nbf x nmos, column-major).
+int launch_std_orbitals(const DevBasis& B, const double* mo, int nmos, int pld, int* fn_shell, double* Ct,
+                        cudaStream_t s);
 
-// Raw[(k0 + kk) + naux * (p(p+1)/2 + q)] = Res[(kk * nmos + p) + nk * nmos * q], q <= p.
-int launch_std_pack(const double* Res, int nk, int nmos, int k0, int naux, double* Raw,
+// First half-transformation of intor_df2c_mo (std/intor.f90:207-261) over the
+// block matrix I of nk auxiliary columns (ld even, >= nk):
+// W[(nu * nmos + p) * ld + k] = sum_a skip(sum_(i in a) C[i, p] (i nu|k)).
+struct StdHalfArgs {
+  DevBasis B;
+  const double* Qab = nullptr;
+  const int* row0 = nullptr;      // pair -> first row of I, -1: none
+  const int* fn_shell = nullptr;
+  const double* col_Q = nullptr;  // Schwarz value of each of the nk columns
+  double thresh = 0.0;
+  const double* I = nullptr;
+  const double* Ct = nullptr;
+  int nk = 0, ld = 0, pld = 0, nmos = 0;  // pld: multiple of 16 std_half_pt(nmos)
+  double* W = nullptr;
+};
+int std_half_pt(int nmos);
+int launch_std_half(const StdHalfArgs& h, cudaStream_t s);
+
+// Raw[col_fn[k] + naux * (p(p+1)/2 + q)] = Res[k + ld * (p + nmos * q)], k < nk, q <= p.
+int launch_std_pack(const double* Res, int nk, int ld, int nmos, const int* col_fn, int naux, double* Raw,
                     cudaStream_t s);
 
 // out[kp * nshells_aux + c] = ||(ab|c)||_2 for pair rec_pair[kp] (kp < npairs)

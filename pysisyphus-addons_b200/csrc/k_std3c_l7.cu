@@ -1,0 +1,4 @@
+// Explicit (ab|c) block kernels of the bra class L_ab = 7 (every auxiliary L).
+#include "k_std3c_impl.cuh"
+
+PA_STD3C_ROW(7)

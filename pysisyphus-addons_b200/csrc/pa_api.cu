@@ -10,6 +10,7 @@
 //   B = L^-1 df (blocked forward substitution) [-> Coulomb tensor]
 #include <cub/device/device_reduce.cuh>
 #include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_scan.cuh>
 
 #include <algorithm>
 #include <limits>
@@ -36,6 +37,7 @@
 #include "k_integrals.cuh"
 #include "k_linalg.cuh"
 #include "k_std.cuh"
+#include "k_std3c.cuh"
 #include "pa_b200.h"
 #include "pa_internal.h"
 
@@ -385,6 +387,7 @@ struct pa_basis_s {
   int* d_class_unit = nullptr;   // units grouped by Lab
   int* d_class_off = nullptr;    // [lab_max + 2]
   int* d_class_pair = nullptr;   // pairs grouped by Lab
+  int* d_pair_class_off = nullptr;  // [lab_max + 2]
   int* d_aux_shell = nullptr;    // aux shells grouped by L
   int* d_aux_off = nullptr;      // [lc_max + 2]
   // QVL screener data: per shell (as an auxiliary basis) and per shell pair
@@ -420,7 +423,8 @@ struct Ctx {
   static constexpr int kNs3c = 4;
   cudaStream_t s3c[kNs3c] = {};
   cudaEvent_t j3c[kNs3c] = {};
-  int* h_info = nullptr;  // pinned
+  int* h_info = nullptr;  // pinned, kHostInfo entries
+  static constexpr int kHostInfo = 32;
   // Stream-ordered pool of the host-buffer entry points (densities, df, R).
   // Freed blocks stay mapped in this private pool, so repeated calls of the
   // same size do not map device memory again; the device's default pool and
@@ -512,7 +516,7 @@ int current_ctx(Ctx** out, DeviceTables* dt) {
     }
     PA_CUDA(cudaEventCreate(&c->m0));
     PA_CUDA(cudaEventCreate(&c->m1));
-    PA_CUDA(cudaMallocHost(&c->h_info, sizeof(int) * 4));
+    PA_CUDA(cudaMallocHost(&c->h_info, sizeof(int) * Ctx::kHostInfo));
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -638,9 +642,10 @@ struct DfBuffers {
   std::vector<ClassRun> runs;
 };
 
-size_t cub_temp_bytes(const pa_basis_s* orb, const pa_basis_s* aux) {
+// Scratch of the CUB calls over lists of n1 and n2 entries.
+size_t cub_temp_bytes(int n1, int n2) {
   size_t need = 0;
-  for (const int n : {orb->pairs.nunits, static_cast<int>(aux->host.shells.size())}) {
+  for (const int n : {n1, n2}) {
     size_t b1 = 0, b2 = 0, b3 = 0;
     cub::DeviceRadixSort::SortPairsDescending(nullptr, b1, (const double*)nullptr, (double*)nullptr,
                                               (const int*)nullptr, (int*)nullptr, n, 0, 64);
@@ -722,7 +727,7 @@ void layout_df(Carver& c, const pa_basis_s* orb, const pa_basis_s* aux, int nd, 
   b->sort_j2 = c.take<int>(nsort);
   b->sort_c = c.take<unsigned char>(nsort);
   b->sort_c2 = c.take<unsigned char>(nsort);
-  b->cub_bytes = cub_temp_bytes(orb, aux);
+  b->cub_bytes = cub_temp_bytes(P.nunits, nx);
   b->cub_tmp = c.take<char>(b->cub_bytes);
   // partial slabs; the work-item granularity grows with the system size (on
   // B200, with every item a chunk of its tile's surviving units: 2 items per
@@ -1111,6 +1116,7 @@ int ensure_pairs(pa_basis b) {
     b->d_class_unit = cnt.take<int>(P.class_unit.size());
     b->d_class_off = cnt.take<int>(P.class_off.size());
     b->d_class_pair = cnt.take<int>(P.class_pair.size());
+    b->d_pair_class_off = cnt.take<int>(P.pair_class_off.size());
   }
   std::vector<char> stage(cnt.used);
   auto put = [&](const void* dst, const void* src, size_t bytes) {
@@ -1124,6 +1130,7 @@ int ensure_pairs(pa_basis b) {
   put(b->d_class_unit, P.class_unit.data(), sizeof(int) * P.class_unit.size());
   put(b->d_class_off, P.class_off.data(), sizeof(int) * P.class_off.size());
   put(b->d_class_pair, P.class_pair.data(), sizeof(int) * P.class_pair.size());
+  put(b->d_pair_class_off, P.pair_class_off.data(), sizeof(int) * P.pair_class_off.size());
   const cudaError_t e = cudaMemcpy(dpair, stage.data(), cnt.used, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(dpair);
@@ -1661,8 +1668,47 @@ int df_host(pa_basis orb, pa_basis aux, int ndens, int nbf, const double* dens, 
 // (nbf x nbf), 2 = df2c_mo (nmos(nmos+1)/2 x naux); all column-major.
 enum StdKind { kStdDf1c = 0, kStdEri2c = 1, kStdDf2cMo = 2 };
 
-// Doubles of W per batch of the df2c_mo half transformation (1 GiB).
+// Limits of one auxiliary batch of df2c_mo, doubles: the block matrix (2 GiB)
+// and its half-transformed form W (1 GiB).
+constexpr size_t kStdBlockBudget = size_t(1) << 28;
 constexpr size_t kStdWBudget = size_t(1) << 27;
+
+// Block kernels of one launch set (k_std3c): every (L_ab, L_c) class with bra
+// entries bra[lab] and the sorted auxiliary slots [s0, s1), spread over the
+// class streams; joined on s.
+struct Std3cBra {
+  const int* list = nullptr;
+  int n = 0;
+};
+int std_blocks(Ctx* c, const pa_basis_s* aux, Std3cArgs a, const std::vector<Std3cBra>& bra, const int* sorted_aux,
+               int s0, int s1, cudaStream_t s, int* launches) {
+  PA_CUDA(cudaEventRecord(c->fork, s));
+  for (int i = 0; i < Ctx::kNs3c; ++i) PA_CUDA(cudaStreamWaitEvent(c->s3c[i], c->fork, 0));
+  const AuxLists& X = aux->aux;
+  int next = 0;
+  // highest L_c and L_ab first: the longest blocks start early
+  for (int lc = X.lc_max; lc >= 0; --lc) {
+    const int b0 = std::max(s0, X.class_off[lc]), b1 = std::min(s1, X.class_off[lc + 1]);
+    if (b1 <= b0) continue;
+    int col = 0;  // columns of the launch's slots below b0
+    for (int l = 0; l < lc; ++l)
+      col += std::max(0, std::min(s1, X.class_off[l + 1]) - std::max(s0, X.class_off[l])) * (2 * l + 1);
+    for (int lab = static_cast<int>(bra.size()) - 1; lab >= 0; --lab) {
+      if (bra[lab].n <= 0) continue;
+      a.bra = bra[lab].list;
+      a.n_bra = bra[lab].n;
+      a.aux = sorted_aux + b0;
+      a.n_aux = b1 - b0;
+      a.col0 = col;
+      *launches += launch_std3c_class(lab, lc, a, c->s3c[next++ % Ctx::kNs3c]);
+    }
+  }
+  for (int i = 0; i < Ctx::kNs3c; ++i) {
+    PA_CUDA(cudaEventRecord(c->j3c[i], c->s3c[i]));
+    PA_CUDA(cudaStreamWaitEvent(s, c->j3c[i], 0));
+  }
+  return PA_OK;
+}
 
 int std_device(pa_basis orb, pa_basis aux, int kind, int nmos, const double* d_mo, double* d_out,
                cudaStream_t s) {
@@ -1683,38 +1729,37 @@ int std_device(pa_basis orb, pa_basis aux, int kind, int nmos, const double* d_m
   const int nx = static_cast<int>(aux->host.shells.size());
   const long long npack = static_cast<long long>(nmos) * (nmos + 1) / 2;
   const long long ncols = kind == kStdDf2cMo ? npack : nbf;
-  // auxiliary shell batches of the df2c_mo half transformation
-  std::vector<int> batch{0};
-  size_t wmax = 0, resmax = 0;
-  if (kind == kStdDf2cMo && nmos > 0) {
-    const size_t per_fn = static_cast<size_t>(nmos) * nbf;
-    size_t fns = 0;
-    for (int i = 0; i < nx; ++i) {
-      const size_t f = 2 * aux->host.shells[i].L + 1;
-      if (fns > 0 && (fns + f) * per_fn > kStdWBudget) {
-        batch.push_back(i);
-        fns = 0;
-      }
-      fns += f;
-      wmax = std::max(wmax, fns * per_fn);
-      resmax = std::max(resmax, fns * static_cast<size_t>(nmos) * nmos);
-    }
+  const bool mo2c = kind == kStdDf2cMo && nmos > 0 && nx > 0 && nbf > 0;
+  const int npairs = P.npairs;
+  // df2c_mo: rows of the block matrix with every pair present, widest shell
+  size_t rows_all = 0, ncmax = 1;
+  size_t i_max = 0, w_max = 0, res_max = 0;
+  const int pld = mo2c ? (nmos + 16 * std_half_pt(nmos) - 1) / (16 * std_half_pt(nmos)) * 16 * std_half_pt(nmos) : 0;
+  if (mo2c) {
+    for (const int2& ab : P.pair_ab)
+      rows_all += static_cast<size_t>(2 * orb->host.shells[ab.x].L + 1) * (2 * orb->host.shells[ab.y].L + 1);
+    ncmax = 2 * static_cast<size_t>(aux->host.lmax) + 1;
+    const size_t cols = static_cast<size_t>(naux) + 1, least = ncmax + 1;  // column counts are rounded up to even
+    i_max = std::max(std::min(kStdBlockBudget, rows_all * cols), rows_all * least);
+    w_max = std::max(std::min(kStdWBudget, static_cast<size_t>(nmos) * nbf * cols),
+                     static_cast<size_t>(nmos) * nbf * least);
+    res_max = w_max / nbf * nmos;
   }
-  batch.push_back(nx);
   Carver cnt;
   // one layout, carved twice (count, then real)
   struct Bufs {
-    double *Qab, *Qc, *esph, *M, *lawork, *raw, *y, *W, *res;
+    double *Qab, *Qc, *esph, *M, *lawork, *raw, *y, *W, *res, *I, *Ct, *keys, *pair_Q, *aux_Q, *col_Q, *qmax;
     double4* pP;
-    int* info;
+    int *info, *vals, *pair, *sorted_aux, *size, *first, *row0, *col_fn, *fn_shell, *nclass;
   } b{};
+  DfBuffers sb;  // sort scratch
   for (int pass = 0; pass < 2; ++pass) {
     Carver cv;
     if (pass == 1) {
       PA_CUDA(c->arena.reserve(cnt.used));
       cv.base = c->arena.base;
     }
-    b.Qab = cv.take<double>(P.npairs);
+    b.Qab = cv.take<double>(npairs);
     b.Qc = cv.take<double>(nx);
     b.pP = cv.take<double4>(P.nunits);
     b.esph = cv.take<double>(P.esph_total);
@@ -1723,8 +1768,39 @@ int std_device(pa_basis orb, pa_basis aux, int kind, int nmos, const double* d_m
     b.info = cv.take<int>(4);
     b.raw = cv.take<double>(static_cast<size_t>(naux) * ncols);
     b.y = cv.take<double>(static_cast<size_t>(naux) * ncols);
-    b.W = cv.take<double>(wmax);
-    b.res = cv.take<double>(resmax);
+    if (mo2c) {
+      const int nsort = std::max(npairs, nx);
+      b.W = cv.take<double>(w_max);
+      b.res = cv.take<double>(res_max);
+      b.I = cv.take<double>(i_max);
+      b.Ct = cv.take<double>(static_cast<size_t>(nbf) * pld);
+      b.keys = cv.take<double>(nsort);
+      b.vals = cv.take<int>(nsort);
+      b.pair_Q = cv.take<double>(npairs);
+      b.pair = cv.take<int>(npairs);
+      b.aux_Q = cv.take<double>(nx);
+      b.sorted_aux = cv.take<int>(nx);
+      b.col_Q = cv.take<double>(naux);
+      b.col_fn = cv.take<int>(naux);
+      b.qmax = cv.take<double>(1);
+      b.size = cv.take<int>(npairs);
+      b.first = cv.take<int>(npairs);
+      b.row0 = cv.take<int>(npairs);
+      b.fn_shell = cv.take<int>(nbf);
+      b.nclass = cv.take<int>(Ctx::kHostInfo);
+      sb.sort_k = cv.take<double>(nsort);
+      sb.sort_p = cv.take<int>(nsort);
+      sb.sort_j = cv.take<int>(nsort);
+      sb.sort_j2 = cv.take<int>(nsort);
+      sb.sort_c = cv.take<unsigned char>(nsort);
+      sb.sort_c2 = cv.take<unsigned char>(nsort);
+      if (pass == 0) {
+        size_t scan = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, scan, (const int*)nullptr, (int*)nullptr, npairs);
+        sb.cub_bytes = std::max(scan, cub_temp_bytes(npairs, nx));
+      }
+      sb.cub_tmp = cv.take<char>(sb.cub_bytes);
+    }
     if (pass == 0) cnt = cv;
   }
   PA_CUDA(cudaEventRecord(c->ev0, s));
@@ -1764,23 +1840,111 @@ int std_device(pa_basis orb, pa_basis aux, int kind, int nmos, const double* d_m
   a.Qab = b.Qab;
   a.Qc = b.Qc;
   const size_t raw_bytes = sizeof(double) * static_cast<size_t>(naux) * ncols;
+  Std3cArgs blk;
+  blk.x.X = aux->dev;
+  blk.x.dt = dt;
+  blk.x.boys_mode = o.boys_mode;
+  blk.x.thresh = o.screen_thresh;
+  blk.B = orb->dev;
+  blk.pair_ab = orb->d_pair_ab;
+  blk.pair_unit0 = orb->d_pair_unit0;
+  blk.unit_pP = b.pP;
+  blk.esph = b.esph;
+  blk.unit_esph = orb->d_unit_esph;
+  blk.Qab = b.Qab;
+  blk.Qc = b.Qc;
   if (kind != kStdDf2cMo) {
-    // screened (a, a, c) entries stay zero (the reference's output starts zeroed)
-    if (raw_bytes) PA_CUDA(cudaMemsetAsync(b.raw, 0, raw_bytes, s));
-    launches += launch_std_df1c(a, b.raw, s);
-  } else if (nmos > 0) {
-    for (size_t bi = 0; bi + 1 < batch.size(); ++bi) {
-      const int c0 = batch[bi], c1 = batch[bi + 1];
-      if (c1 <= c0) continue;
-      const int k0 = aux->host.shells[c0].sph_off;
-      const int k1 = c1 < nx ? aux->host.shells[c1].sph_off : naux;
-      const int nk = k1 - k0;
-      launches += launch_std_df2c_half(a, c0, c1, k0, nmos, d_mo, b.W, s);
-      // Res[(kk, p), q] = sum_nu W[(kk, p)][nu] C[nu, q] (std/intor.f90:263-279)
-      launches += gemm(true, false, nk * nmos, nmos, nbf, 1.0, b.W, nbf, d_mo, nbf, 0.0, b.res,
-                       static_cast<long long>(nk) * nmos, false, s);
-      launches += launch_std_pack(b.res, nk, nmos, k0, naux, b.raw, s);
+    // (mu mu|P): the shells grouped by L, L_ab = 2 L; every entry is written
+    // (screened (a, a, c) entries as zero)
+    blk.diag = 1;
+    blk.out = b.raw;
+    blk.ld = naux;
+    std::vector<Std3cBra> bra(P.lab_max + 1);
+    for (int l = 0; 2 * l <= P.lab_max && l <= orb->aux.lc_max; ++l) {
+      bra[2 * l].list = orb->d_aux_shell + orb->aux.class_off[l];
+      bra[2 * l].n = orb->aux.class_off[l + 1] - orb->aux.class_off[l];
     }
+    st = std_blocks(c, aux, blk, bra, aux->d_aux_shell, 0, nx, s, &launches);
+    if (st != PA_OK) return st;
+  } else if (mo2c) {
+    // layout of the block matrix: pairs and auxiliary shells sorted by Schwarz
+    // value within their class, rows for the pairs that meet the largest Q_c
+    k_gather_aux_keys<<<(nx + 255) / 256, 256, 0, s>>>(nx, aux->d_aux_shell, b.Qc, aux->dev.shell, nullptr, 1.0,
+                                                       b.keys, b.vals);
+    size_t bytes = sb.cub_bytes;
+    PA_CUDA(cub::DeviceReduce::Max(sb.cub_tmp, bytes, b.keys, b.qmax, nx, s));
+    launches += 2;
+    launches += class_sort_desc(sb, b.keys, b.vals, aux->d_aux_shell, aux->d_aux_off, aux->aux.lc_max + 1, nx, b.aux_Q,
+                                b.sorted_aux, s);
+    launches += launch_std_columns(nx, b.sorted_aux, b.aux_Q, aux->d_aux_off, aux->aux.lc_max + 1, aux->dev.shell,
+                                   b.col_fn, b.col_Q, s);
+    launches += launch_std_orbitals(orb->dev, d_mo, nmos, pld, b.fn_shell, b.Ct, s);
+    int* h = c->h_info;
+    static_assert(2 * PA_LMAX + 2 <= Ctx::kHostInfo, "class counts and the row total fit the pinned buffer");
+    PA_CUDA(cudaMemsetAsync(b.nclass, 0, sizeof(int) * Ctx::kHostInfo, s));
+    if (npairs > 0) {
+      launches += launch_std_pair_keys(npairs, orb->d_class_pair, b.Qab, b.keys, b.vals, s);
+      launches += class_sort_desc(sb, b.keys, b.vals, orb->d_class_pair, orb->d_pair_class_off, P.lab_max + 1, npairs,
+                                  b.pair_Q, b.pair, s);
+      launches += launch_std_pair_size(a, npairs, b.pair_Q, b.pair, orb->d_pair_class_off, P.lab_max + 1, b.qmax,
+                                       b.size, b.nclass, s);
+      bytes = sb.cub_bytes;
+      PA_CUDA(cub::DeviceScan::ExclusiveSum(sb.cub_tmp, bytes, b.size, b.first, npairs, s));
+      ++launches;
+      launches += launch_std_pair_row(npairs, b.pair, b.size, b.first, b.row0, b.nclass + 2 * PA_LMAX + 1, s);
+    }
+    PA_CUDA(cudaMemcpyAsync(h, b.nclass, sizeof(int) * (2 * PA_LMAX + 2), cudaMemcpyDeviceToHost, s));
+    PA_CUDA(cudaStreamSynchronize(s));
+    const size_t rows = static_cast<size_t>(h[2 * PA_LMAX + 1]);
+    std::vector<Std3cBra> bra(P.lab_max + 1);
+    for (int lab = 0; lab <= P.lab_max; ++lab) {
+      bra[lab].list = b.pair + P.pair_class_off[lab];
+      bra[lab].n = h[lab];
+    }
+    blk.row0 = b.row0;
+    blk.out = b.I;
+    StdHalfArgs hf;
+    hf.B = orb->dev;
+    hf.Qab = b.Qab;
+    hf.row0 = b.row0;
+    hf.fn_shell = b.fn_shell;
+    hf.thresh = o.screen_thresh;
+    hf.I = b.I;
+    hf.Ct = b.Ct;
+    hf.pld = pld;
+    hf.nmos = nmos;
+    hf.W = b.W;
+    // batches of sorted auxiliary slots: as many columns as both buffers hold
+    const size_t col_cap = std::min(i_max / std::max<size_t>(rows, 1), w_max / (static_cast<size_t>(nmos) * nbf));
+    const AuxLists& X = aux->aux;
+    int s0 = 0, k0 = 0;
+    while (s0 < nx) {
+      int s1 = s0, L = 0;
+      size_t nk = 0;
+      while (s1 < nx) {
+        while (s1 >= X.class_off[L + 1]) ++L;
+        const size_t more = nk + 2 * L + 1;
+        if (s1 > s0 && (more + 1) / 2 * 2 > col_cap) break;
+        nk = more;
+        ++s1;
+      }
+      const int ld = static_cast<int>((nk + 1) / 2 * 2);
+      blk.ld = ld;
+      st = std_blocks(c, aux, blk, bra, b.sorted_aux, s0, s1, s, &launches);
+      if (st != PA_OK) return st;
+      hf.col_Q = b.col_Q + k0;
+      hf.nk = static_cast<int>(nk);
+      hf.ld = ld;
+      launches += launch_std_half(hf, s);
+      // Res[(p, k), q] = sum_nu W[nu][(p, k)] C[nu, q] (std/intor.f90:263-279)
+      launches += gemm(false, false, ld * nmos, nmos, nbf, 1.0, b.W, static_cast<long long>(ld) * nmos, d_mo, nbf, 0.0,
+                       b.res, static_cast<long long>(ld) * nmos, false, s);
+      launches += launch_std_pack(b.res, static_cast<int>(nk), ld, nmos, b.col_fn + k0, naux, b.raw, s);
+      s0 = s1;
+      k0 += static_cast<int>(nk);
+    }
+  } else if (raw_bytes) {
+    PA_CUDA(cudaMemsetAsync(b.raw, 0, raw_bytes, s));  // no orbital functions
   }
   PA_CUDA(cudaEventRecord(c->ph[1], s));
   PA_CUDA(cudaStreamWaitEvent(s, c->m1, 0));

@@ -15,6 +15,7 @@
 
 #include "boys.cuh"
 #include "k_df3c.cuh"
+#include "k_std3c.cuh"
 #include "pa_internal.h"
 #include "sph_raw.cuh"
 
@@ -213,6 +214,7 @@ int build_tables(TablesOnDevice* out, std::string* err) {
   dt.sum_idx = reinterpret_cast<const int16_t*>(put(sum_idx.data(), sizeof(int16_t) * sum_idx.size()));
   dt.rdesc = reinterpret_cast<const int*>(put(rdesc.data(), sizeof(int) * rdesc.size()));
   e = upload_sph_rownorm(rownorm.data(), 0);
+  if (e == cudaSuccess) e = upload_std3c_rownorm(rownorm.data(), 0);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     *err = std::string("table upload: ") + cudaGetErrorString(e);
