@@ -1,8 +1,8 @@
 // Dense FP64 linear algebra of the density-fitting path (column-major):
 //  * blocked right-looking Cholesky of the metric, lower triangle
-//    (replaces dpotrf("L"), common/linalg.f90:78); each 64 x 64 diagonal block is
-//    factorized and inverted by one thread block, the panel below it is
-//    scaled in place and the trailing matrix updated by a lower GEMM;
+//    (replaces dpotrf("L"), common/linalg.f90:78); one launch per 64 columns takes
+//    the panel and the next diagonal block with its inverse, another the
+//    trailing matrix beside the next step;
 //  * L^-1 df as a blocked forward substitution on the density columns, using
 //    the inverted diagonal blocks (replaces dtrtri("L","N"), common/linalg.f90:81,
 //    followed by dtrmm("L","L","N","N"), diabatization/intor.f90:198: the
@@ -17,6 +17,7 @@
 #include "k_linalg.cuh"
 
 #include <cstdint>
+#include <type_traits>
 
 namespace pa {
 
@@ -24,32 +25,39 @@ namespace {
 
 constexpr int NB = 64;
 
-// Factorize the nb x nb diagonal block at (j0, j0) in place (lower) and write
-// its inverse (lower, zeros above the diagonal, NB x NB) to dinv. The serial
-// part is kept short: one square root and one reciprocal per pivot, the
-// columns scaled by the reciprocal (as dpotf2 does), rows held in registers.
-//  * Cholesky, per 16-column sub-block: warp 0 factors the 16 x 16 diagonal
-//    sub-block (lane r holds row r, pivots and L(j, k) move by shuffles); one
-//    thread per row below solves x L11^T = a in registers; all threads update
-//    the trailing lower triangle;
-//  * inverse: four warps invert the diagonal sub-blocks (lane c holds column c
-//    in registers), then block rows i = 1..3 follow from
-//    X_ij = -X_ii sum_(j <= k < i) L_ik X_kj.
+__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ void cp_async8(double* smem_dst, const double* gmem_src) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem_src));
+}
+
+__device__ __forceinline__ void cp_async16_ld(double* smem_dst, const double* gmem_src) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src));
+}
+
+// Cholesky factor of the 64 x 64 block S (lower triangle; row stride NB + 1) in
+// place, its inverse in X (zeros above the diagonal), T scratch; all 256
+// threads, S complete on entry (after a barrier). Rows and columns from nb on
+// hold the identity. The serial chain is kept short: per pivot one reciprocal
+// square root (the pivot's root follows from it and one Newton correction), per
+// 16-column sub-block
+//  * warp 0 factors the 16 x 16 diagonal sub-block (lane r holds row r, pivots
+//    and L(j, k) move by shuffles);
+//  * one thread per row below solves x L11^T = a in registers;
+//  * all threads update the trailing lower triangle.
+// Inverse: four warps invert the diagonal sub-blocks (lane c holds column c,
+// right-looking, so a row's updates are independent), then the off-diagonal
+// blocks follow by doubling: X_21 = -X_22 (L_21 X_11) at 16 and at 32 columns.
 constexpr int SB = 16;
-__global__ void __launch_bounds__(256) k_potrf_diag_inv(double* A, long long lda, int j0, int nb,
-                                                        double* dinv, int* info) {
-  extern __shared__ double dsm[];
-  double(*S)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm);                       // the block, then L
-  double(*Xs)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm + NB * (NB + 1));      // L^-1
-  double(*Ts)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm + 2 * NB * (NB + 1));  // block-row sums
-  __shared__ double invd[NB];                                                           // 1 / L(j, j)
+__device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X)[NB + 1], double (*T)[NB + 1],
+                                                 double* invd, int nb, int pivot0, int* info) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int idx = tid; idx < NB * NB; idx += 256) {
-    const int r = idx & (NB - 1), c = idx >> 6;
-    S[r][c] = (r < nb && c < nb) ? (c <= r ? A[(j0 + r) + lda * (j0 + c)] : 0.0) : (r == c ? 1.0 : 0.0);
-    Xs[r][c] = 0.0;
-  }
-  __syncthreads();
   for (int k0 = 0; k0 < NB; k0 += SB) {
     if (warp == 0) {
       // lanes 16..31 repeat lanes 0..15 (they only feed the shuffles)
@@ -61,12 +69,10 @@ __global__ void __launch_bounds__(256) k_potrf_diag_inv(double* A, long long lda
       for (int k = 0; k < SB; ++k) {
         double dkk = __shfl_sync(0xffffffffu, v[k], k);
         if (!(dkk > 0.0)) {
-          if (lane == 0 && k0 + k < nb) atomicCAS(info, 0, j0 + k0 + k + 1);
+          if (lane == 0 && k0 + k < nb) atomicCAS(info, 0, pivot0 + k0 + k + 1);
           dkk = 1.0;  // keep the factor finite; the error is reported through info
         }
-        const double d = sqrt(dkk);
-        const double id = 1.0 / d;
-        if (r == k) v[k] = d;
+        const double id = rsqrt(dkk);
         if (r > k) v[k] *= id;  // L(r, k)
 #pragma unroll
         for (int j = 1; j < SB; ++j) {  // fixed trip count: j > k folds once k is unrolled
@@ -74,6 +80,10 @@ __global__ void __launch_bounds__(256) k_potrf_diag_inv(double* A, long long lda
           const double ljk = __shfl_sync(0xffffffffu, v[k], j);  // L(j, k) from lane j
           if (r >= j) v[j] = fma(-v[k], ljk, v[j]);
         }
+        // sqrt(dkk) from its reciprocal: off the chain of the next pivot
+        const double d0 = dkk * id;
+        const double d = isinf(dkk) ? dkk : fma(fma(-d0, d0, dkk), 0.5 * id, d0);
+        if (r == k) v[k] = d;
         if (lane == k) invd[k0 + k] = id;
       }
       if (lane < SB) {
@@ -100,106 +110,248 @@ __global__ void __launch_bounds__(256) k_potrf_diag_inv(double* A, long long lda
       for (int j = 0; j < SB; ++j) S[pr][k0 + j] = v[j];
     }
     __syncthreads();
-    // trailing lower triangle: S[r][c] -= sum_k S[r][k] S[c][k], k in the sub-block
-    const int m = NB - k0 - SB;
-    for (int e = tid; e < m * m; e += 256) {
-      const int rr = k0 + SB + e / m, cc = k0 + SB + e % m;
-      if (cc > rr) continue;
-      double v = S[rr][cc];
+    // trailing lower triangle: S[r][c] -= sum_k S[r][k] S[c][k], k in the
+    // sub-block; a thread per entry of each 16 x 16 tile
+    const int ty = tid >> 4, tx = tid & 15;
+    for (int r0 = k0 + SB; r0 < NB; r0 += SB)
+      for (int c0 = k0 + SB; c0 <= r0; c0 += SB) {
+        const int rr = r0 + ty, cc = c0 + tx;
+        if (cc > rr) continue;
+        double v0 = 0.0, v1 = 0.0;
 #pragma unroll
-      for (int k = 0; k < SB; ++k) v = fma(-S[rr][k0 + k], S[cc][k0 + k], v);
-      S[rr][cc] = v;
-    }
+        for (int k = 0; k < SB; k += 2) {
+          v0 = fma(S[rr][k0 + k], S[cc][k0 + k], v0);
+          v1 = fma(S[rr][k0 + k + 1], S[cc][k0 + k + 1], v1);
+        }
+        S[rr][cc] -= v0 + v1;
+      }
     __syncthreads();
   }
-  // write the factor back
-  for (int idx = tid; idx < NB * NB; idx += 256) {
-    const int r = idx & (NB - 1), c = idx >> 6;
-    if (r < nb && c <= r) A[(j0 + r) + lda * (j0 + c)] = S[r][c];
-  }
-  // diagonal sub-blocks of the inverse: warp w < 4 inverts sub-block w by
-  // forward substitution, lane c holding column c
+  for (int idx = tid; idx < NB * NB; idx += 256) X[idx >> 6][idx & (NB - 1)] = 0.0;
+  __syncthreads();
   if (warp < NB / SB) {
     const int o = warp * SB, c = lane & (SB - 1);
     double x[SB];
 #pragma unroll
-    for (int i = 0; i < SB; ++i) {
-      double v = (i == c) ? 1.0 : 0.0;
+    for (int i = 0; i < SB; ++i) x[i] = (i == c) ? 1.0 : 0.0;
 #pragma unroll
-      for (int k = 0; k < SB - 1; ++k)
-        if (k < i) v = fma(-S[o + i][o + k], x[k], v);
-      x[i] = (i >= c) ? v * invd[o + i] : 0.0;
+    for (int i = 0; i < SB; ++i) {
+      x[i] *= invd[o + i];
+#pragma unroll
+      for (int k = 1; k < SB; ++k)
+        if (k > i) x[k] = fma(-S[o + k][o + i], x[i], x[k]);
     }
     if (lane < SB) {
 #pragma unroll
-      for (int i = 0; i < SB; ++i) Xs[o + i][o + c] = x[i];
+      for (int i = 0; i < SB; ++i)
+        if (i >= c) X[o + i][o + c] = x[i];
     }
   }
   __syncthreads();
-  // block rows i = 1..3: T_j = sum_(j <= k < i) L_ik X_kj, then X_ij = -X_ii T_j
-  for (int bi = 1; bi < NB / SB; ++bi) {
-    const int ro = bi * SB, ncol = bi * SB;  // columns 0 .. ro - 1
-    for (int e = tid; e < SB * ncol; e += 256) {
-      const int i = e / ncol, c = e % ncol;
-      const int bj = c / SB;
-      double v = 0.0;
-      for (int k = bj * SB; k < ro; ++k) v = fma(S[ro + i][k], Xs[k][c], v);
-      Ts[ro + i][c] = v;
+  // doubling: blocks of w columns, T = L_21 X_11 (X_11 lower triangular), then
+  // X_21 = -X_22 T; every sum in two interleaved halves
+  auto level = [&](auto wc) {
+    constexpr int w = decltype(wc)::value;
+    constexpr int npair = NB / (2 * w), per = npair * w * w / 256;
+#pragma unroll
+    for (int q = 0; q < per; ++q) {
+      const int e = tid + 256 * q;
+      const int pairi = e / (w * w), i = (e / w) % w, j = e % w, o = pairi * 2 * w;
+      double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+      for (int k = 0; k < w; k += 2) {
+        v0 = fma(S[o + w + i][o + k], X[o + k][o + j], v0);
+        v1 = fma(S[o + w + i][o + k + 1], X[o + k + 1][o + j], v1);
+      }
+      T[o + w + i][j] = v0 + v1;
     }
     __syncthreads();
-    for (int e = tid; e < SB * ncol; e += 256) {
-      const int i = e / ncol, c = e % ncol;
-      double v = 0.0;
-      for (int k = 0; k <= i; ++k) v = fma(Xs[ro + i][ro + k], Ts[ro + k][c], v);
-      Xs[ro + i][c] = -v;
+#pragma unroll
+    for (int q = 0; q < per; ++q) {
+      const int e = tid + 256 * q;
+      const int pairi = e / (w * w), i = (e / w) % w, j = e % w, o = pairi * 2 * w;
+      double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+      for (int k = 0; k < w; k += 2) {
+        v0 = fma(X[o + w + i][o + w + k], T[o + w + k][j], v0);
+        v1 = fma(X[o + w + i][o + w + k + 1], T[o + w + k + 1][j], v1);
+      }
+      X[o + w + i][o + j] = -(v0 + v1);
     }
     __syncthreads();
-  }
-  for (int idx = tid; idx < NB * NB; idx += 256) {
-    const int r = idx & (NB - 1), c = idx >> 6;
-    dinv[r + NB * c] = (r < nb && c <= r) ? Xs[r][c] : 0.0;
+  };
+  level(std::integral_constant<int, SB>{});
+  level(std::integral_constant<int, 2 * SB>{});
+}
+
+// acc += A^T-layout tile product over [0, kq): As[k][row], Bs[k][col] with row
+// stride kPanLd; warp w owns rows 16 (w % 4) and columns 32 (w / 4).
+constexpr int kPanLd = NB + 4;  // 4 (mod 16): conflict-free m8n8k4 fragment loads
+__device__ __forceinline__ void panel_mma(double (&acc)[2][4][2], const double* As, const double* Bs, int kq) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int wm = (warp & 3) * 16, wn = (warp >> 2) * 32;
+#pragma unroll 4
+  for (int q = 0; q < kq; q += 4) {
+    double a[2], b[4];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) a[mt] = As[(q + t4) * kPanLd + wm + 8 * mt + g];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) b[nt] = Bs[(q + t4) * kPanLd + wn + 8 * nt + g];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) dmma_m8n8k4(acc[mt][nt][0], acc[mt][nt][1], a[mt], b[nt]);
   }
 }
 
-// Panel below the diagonal block (rows j0 + NB.., columns j0..j0 + nb):
-// P := P Dinv^T in place. One block per 64 rows; the whole row slice is read
-// into shared memory before it is overwritten.
-__global__ void __launch_bounds__(256) k_panel_inplace(double* A, long long lda, int j0, int nb,
-                                                       int rows, const double* __restrict__ dinv) {
-  extern __shared__ double psm[];
-  double(*P)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(psm);           // [row][p]
-  double(*D)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(psm + NB * (NB + 1));  // [j][p]
-  const int tid = threadIdx.x;
-  const int i0 = blockIdx.x * NB;
-  double* base = A + (j0 + nb) + lda * j0;
-#pragma unroll
-  for (int idx = tid; idx < NB * NB; idx += 256) {
-    const int i = idx & (NB - 1), p = idx >> 6;
-    P[i][p] = (i0 + i < rows && p < nb) ? base[(i0 + i) + lda * p] : 0.0;
-    D[i][p] = dinv[i + NB * p];
+// One step of the blocked Cholesky factorization: the panel of block column c,
+// and (block 0) the next diagonal block. Block x owns row block i = c + 1 + x:
+//   P(i, c) = (A(i, c) - P(i, c - 1) P(c, c - 1)^T) L(c, c)^-T,
+// and for i = c + 1 then
+//   A(i, i) -= P(i, c - 1) P(i, c - 1)^T + P(i, c) P(i, c)^T, factor, inverse.
+// The contributions of columns below c - 1 came from the trailing updates
+// (k_syrk_update), which leave out what this kernel takes itself: the next
+// block column and the diagonal block after it. So the chain from one
+// diagonal block to the next is one launch, and the trailing update of a step
+// runs beside the next step. c = -1: the first diagonal block alone.
+//
+// Bound: latency. Critical path of a step at 40 atoms (n = 2240): ~25 us, block
+// 0's four 64^3 products and the factor; with a launch each for the factor
+// (40 us), the panel and the next column's update a step took ~100 us.
+constexpr size_t kCholSmem = sizeof(double) * 3 * NB * kPanLd;
+__global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, int n, int c, double* dinv,
+                                                      int* info) {
+  extern __shared__ __align__(16) double csm[];
+  double* As = csm;                    // [p][r] P(i, c - 1), later the inverse
+  double* Bs = As + NB * kPanLd;       // [p][r] P(c, c - 1), later [p][r] of the updated A(i, c), then S
+  double* Ds = Bs + NB * kPanLd;       // [p][j] L(c, c)^-1, later [p][r] P(i, c), then scratch
+  __shared__ double invd[NB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int wm = (warp & 3) * 16, wn = (warp >> 2) * 32;
+  const int i = c + 1 + blockIdx.x, r0 = i * NB, nr = min(NB, n - r0);
+  const bool diag = blockIdx.x == 0;
+  if (c >= 0) {
+    const double* dc = dinv + static_cast<size_t>(c) * NB * NB;
+    for (int idx = tid; idx < NB * NB; idx += 256) {
+      const int r = idx & (NB - 1), p = idx >> 6;
+      if (c > 0) {
+        const double* col = A + lda * ((c - 1) * NB + p);
+        if (r < nr)
+          cp_async8(As + p * kPanLd + r, col + r0 + r);
+        else
+          As[p * kPanLd + r] = 0.0;
+        cp_async8(Bs + p * kPanLd + r, col + c * NB + r);
+      }
+      cp_async8(Ds + p * kPanLd + r, dc + r + NB * p);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
   }
+  // this thread's entries of A(i, c), in flight with the copies
+  double cv[2][4][2];
+  double* Ac = A + r0 + lda * (static_cast<long long>(c) * NB);
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
+        cv[mt][nt][e] = (c >= 0 && r < nr) ? Ac[r + lda * j] : 0.0;
+      }
+  double acc[2][4][2];
+  auto clear = [&] {
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
+  };
+  if (c >= 0) {
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    if (c > 0) {
+      clear();
+      panel_mma(acc, As, Bs, NB);
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) cv[mt][nt][e] -= acc[mt][nt][e];
+      __syncthreads();  // Bs is rewritten
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) Bs[(wn + 8 * nt + 2 * t4 + e) * kPanLd + wm + 8 * mt + g] = cv[mt][nt][e];
+    __syncthreads();
+    clear();
+    panel_mma(acc, Bs, Ds, wn + 32);  // row j of the inverse ends at column j
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
+          if (r < nr) Ac[r + lda * j] = acc[mt][nt][e];
+        }
+    if (!diag) return;
+    __syncthreads();  // Bs and Ds are rewritten
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          Ds[(wn + 8 * nt + 2 * t4 + e) * kPanLd + wm + 8 * mt + g] = acc[mt][nt][e];
+  }
+  // the next diagonal block (rows past n: identity)
+  double* Ai = A + r0 + lda * static_cast<long long>(r0);
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
+        cv[mt][nt][e] = (r < nr && j <= r) ? Ai[r + lda * j] : (r == j ? 1.0 : 0.0);
+      }
   __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
-  double acc[4][4] = {};
-  for (int p = 0; p < NB; ++p) {
-    double x[4], y[4];
+  for (int term = 0; term < 2; ++term) {  // columns c - 1, then c
+    if (c < 1 - term) continue;
+    clear();
+    if (wm + 15 >= wn) panel_mma(acc, term == 0 ? As : Ds, term == 0 ? As : Ds, NB);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      x[u] = P[tx + 16 * u][p];
-      y[u] = D[ty + 16 * u][p];
-    }
+    for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+      for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = fma(x[u], y[v], acc[u][v]);
+        for (int e = 0; e < 2; ++e) cv[mt][nt][e] -= acc[mt][nt][e];
   }
+  double(*S)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(Bs);
+  double(*X)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(As);
+  double(*T)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(Ds);
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int i = i0 + tx + 16 * u, j = ty + 16 * v;
-      if (i < rows && j < nb) base[i + lda * j] = acc[u][v];
-    }
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
+        S[r][j] = j <= r ? cv[mt][nt][e] : 0.0;
+      }
+  __syncthreads();  // As and Ds are free as well
+  factor_invert_64(S, X, T, invd, nr, r0, info);
+  double* di = dinv + static_cast<size_t>(i) * NB * NB;
+  for (int idx = tid; idx < NB * NB; idx += 256) {
+    const int r = idx & (NB - 1), j = idx >> 6;
+    if (r < nr && j <= r) Ai[r + lda * j] = S[r][j];
+    di[r + NB * j] = (r < nr && j <= r) ? X[r][j] : 0.0;
+  }
 }
 
 // Super-step of the blocked forward substitution B := L^-1 B (right-looking)
@@ -310,12 +462,6 @@ __global__ void __launch_bounds__(256) k_trsm_super(const double* __restrict__ L
   }
 }
 
-__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
 // C[m x n] := beta C + alpha op(A) op(B); op(A) is m x k, op(B) is k x n.
 // 64 x 64 tiles, k-steps of 16 staged in shared memory, products on the FP64
 // tensor cores (mma.sync m8n8k4): warp w owns rows 16 (w % 4) .. + 16 and
@@ -400,10 +546,9 @@ __global__ void __launch_bounds__(256) k_gemm(int m, int n, int k, double alpha,
 }
 
 // Trailing update of the Cholesky factorization: C -= P P^T on the lower part
-// (i >= j) of C (m x ncols, ncols <= m, column-major, ldc), P (m x k,
-// column-major, ldp, k <= NB). One block per 64 x 64 tile of that lower part:
-// blockIdx.x enumerates the triangle of the first ncols tile rows, then the
-// full tile rows below. Both panels of a tile are staged whole (every k at
+// (i >= j) of C (m x m, column-major, ldc) without its first 64 x 64 diagonal
+// tile (k_chol_step takes that one), P (m x k, column-major, ldp, k <= NB).
+// One block per 64 x 64 tile of that lower part, row by row. Both panels of a tile are staged whole (every k at
 // once) by cp.async copies (16 bytes when the columns are 16-byte aligned,
 // else 8 bytes: ldp may be odd), in rows of 68 doubles
 // (4 mod 16: conflict-free m8n8k4 fragment loads); two blocks per SM (128
@@ -415,38 +560,21 @@ __global__ void __launch_bounds__(256) k_gemm(int m, int n, int k, double alpha,
 constexpr int kSyrkLd = TM + 4;
 constexpr size_t kSyrkSmem = sizeof(double) * 2 * NB * kSyrkLd;
 
-__device__ __forceinline__ void cp_async8(double* smem_dst, const double* gmem_src) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem_src));
-}
-
-__device__ __forceinline__ void cp_async16_ld(double* smem_dst, const double* gmem_src) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src));
-}
-
 // V16: the panel columns start on 16-byte boundaries (ldp even, P aligned), so
 // pairs of rows are copied 16 bytes at a time. The block's entries of C are
 // loaded into registers before the panels arrive, so their latency overlaps
 // the copies and the products.
 template <bool V16>
-__global__ void __launch_bounds__(256, 2) k_syrk_update(int m, int ncols, int k, const double* __restrict__ P,
+__global__ void __launch_bounds__(256, 2) k_syrk_update(int m, int k, const double* __restrict__ P,
                                                         long long ldp, double* C, long long ldc) {
   extern __shared__ __align__(16) double sm[];
   double* As = sm;                  // As[c * kSyrkLd + r] = P[i0 + r, c]
   double* Bs = sm + NB * kSyrkLd;   // Bs[c * kSyrkLd + r] = P[j0 + r, c]
-  const int nbc = (ncols + TN - 1) / TN;
-  const int t = blockIdx.x, ntri = nbc * (nbc + 1) / 2;
-  int bi, bj;
-  if (t < ntri) {
-    bi = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-    while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
-    while (bi * (bi + 1) / 2 > t) --bi;
-    bj = t - bi * (bi + 1) / 2;
-  } else {
-    bi = nbc + (t - ntri) / nbc;
-    bj = (t - ntri) % nbc;
-  }
+  const int t = blockIdx.x + 1;  // tile (0, 0) is left out
+  int bi = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
+  while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
+  while (bi * (bi + 1) / 2 > t) --bi;
+  const int bj = t - bi * (bi + 1) / 2;
   const int i0 = bi * TM, j0 = bj * TN;
   const int kq = (k + TK - 1) / TK * TK;
   if constexpr (V16) {
@@ -460,10 +588,10 @@ __global__ void __launch_bounds__(256, 2) k_syrk_update(int m, int ncols, int k,
         da[0] = (c < k && i0 + r < m) ? P[(i0 + r) + ldp * c] : 0.0;
         da[1] = 0.0;
       }
-      if (c < k && j0 + r + 1 < ncols) {
+      if (c < k && j0 + r + 1 < m) {
         cp_async16_ld(db, P + (j0 + r) + ldp * c);
       } else {
-        db[0] = (c < k && j0 + r < ncols) ? P[(j0 + r) + ldp * c] : 0.0;
+        db[0] = (c < k && j0 + r < m) ? P[(j0 + r) + ldp * c] : 0.0;
         db[1] = 0.0;
       }
     }
@@ -476,7 +604,7 @@ __global__ void __launch_bounds__(256, 2) k_syrk_update(int m, int ncols, int k,
         cp_async8(da, P + (i0 + r) + ldp * c);
       else
         *da = 0.0;
-      if (c < k && j0 + r < ncols)
+      if (c < k && j0 + r < m)
         cp_async8(db, P + (j0 + r) + ldp * c);
       else
         *db = 0.0;
@@ -495,7 +623,7 @@ __global__ void __launch_bounds__(256, 2) k_syrk_update(int m, int ncols, int k,
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int gi = i0 + wm + 8 * mt + g, gj = j0 + wn + 8 * nt + 2 * t4 + i;
-        cv[mt][nt][i] = (gi < m && gj < ncols && gi >= gj) ? C[gi + ldc * gj] : 0.0;
+        cv[mt][nt][i] = (gi < m && gj < m && gi >= gj) ? C[gi + ldc * gj] : 0.0;
       }
   asm volatile("cp.async.wait_group 0;\n" ::);
   __syncthreads();
@@ -519,7 +647,7 @@ __global__ void __launch_bounds__(256, 2) k_syrk_update(int m, int ncols, int k,
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int gi = i0 + wm + 8 * mt + g, gj = j0 + wn + 8 * nt + 2 * t4 + i;
-        if (gi < m && gj < ncols && gi >= gj) C[gi + ldc * gj] = cv[mt][nt][i] + -1.0 * acc[mt][nt][i];
+        if (gi < m && gj < m && gi >= gj) C[gi + ldc * gj] = cv[mt][nt][i] + -1.0 * acc[mt][nt][i];
       }
 }
 
@@ -565,8 +693,6 @@ __global__ void k_add_diagonal(double* A, int n, double shift) {
   if (i < n) A[i + static_cast<long long>(n) * i] += shift;
 }
 
-constexpr size_t kTileSmem = sizeof(double) * NB * (NB + 1);
-
 int gemm_impl(bool ta, bool tb, int m, int n, int k, double alpha, const double* A, long long lda,
               const double* B, long long ldb, double beta, double* C, long long ldc, bool lower_c,
               bool lower_a, cudaStream_t s) {
@@ -584,16 +710,15 @@ int gemm_impl(bool ta, bool tb, int m, int n, int k, double alpha, const double*
   return 1;
 }
 
-// C -= P P^T on the lower part of C (m x ncols), P m x k (k <= NB).
-int syrk_update(int m, int ncols, int k, const double* P, long long ldp, double* C, long long ldc,
-                cudaStream_t s) {
-  if (m <= 0 || ncols <= 0) return 0;
-  const long long nbr = (m + TM - 1) / TM, nbc = (ncols + TN - 1) / TN;
-  const long long tiles = nbc * (nbc + 1) / 2 + (nbr - nbc) * nbc;
+// C -= P P^T on the lower part of C (m x m) without its first diagonal tile, P m x k (k <= NB).
+int syrk_update(int m, int k, const double* P, long long ldp, double* C, long long ldc, cudaStream_t s) {
+  if (m <= 0) return 0;
+  const long long nbr = (m + TM - 1) / TM, tiles = nbr * (nbr + 1) / 2 - 1;
+  if (tiles <= 0) return 0;
   if (ldp % 2 == 0 && reinterpret_cast<uintptr_t>(P) % 16 == 0)
-    k_syrk_update<true><<<static_cast<unsigned>(tiles), 256, kSyrkSmem, s>>>(m, ncols, k, P, ldp, C, ldc);
+    k_syrk_update<true><<<static_cast<unsigned>(tiles), 256, kSyrkSmem, s>>>(m, k, P, ldp, C, ldc);
   else
-    k_syrk_update<false><<<static_cast<unsigned>(tiles), 256, kSyrkSmem, s>>>(m, ncols, k, P, ldp, C, ldc);
+    k_syrk_update<false><<<static_cast<unsigned>(tiles), 256, kSyrkSmem, s>>>(m, k, P, ldp, C, ldc);
   return 1;
 }
 
@@ -613,47 +738,38 @@ size_t linalg_workspace_doubles(int n) {
 int cholesky_lower(double* A, int n, int* d_info, double* work, cudaStream_t s,
                    const CholLookahead* la) {
   int launches = 0;
-  cudaFuncSetAttribute(k_panel_inplace, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(2 * kTileSmem));
-  cudaFuncSetAttribute(k_potrf_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(3 * kTileSmem));
+  cudaFuncSetAttribute(k_chol_step, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kCholSmem));
   cudaFuncSetAttribute(k_syrk_update<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSyrkSmem));
   cudaFuncSetAttribute(k_syrk_update<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSyrkSmem));
   cudaMemsetAsync(d_info, 0, sizeof(int), s);
   const int nblk = (n + NB - 1) / NB;
-  bool rest_pending = false;  // a trailing update of the previous step is queued on la->aux
-  // per block column b: diagonal factor + inverse, panel P := P L_bb^-T, then
-  // A22 -= P P^T, split (with lookahead) into the next block column (main
-  // stream, on the path to the next diagonal block) and the rest (aux stream)
-  for (int b = 0; b < nblk; ++b) {
-    const int j0 = b * NB, nb = std::min(NB, n - j0);
-    double* Db = work + static_cast<size_t>(b) * NB * NB;
-    k_potrf_diag_inv<<<1, 256, 3 * kTileSmem, s>>>(A, n, j0, nb, Db, d_info);
+  // Step c (k_chol_step) on s; its trailing update of block columns c + 2.. on
+  // the aux stream beside step c + 1, which needs the update of step c - 1 only.
+  bool pending[2] = {false, false};  // an update of a step of this parity is queued on la->aux
+  for (int c = -1; c + 1 < nblk; ++c) {
+    if (la && c >= 1 && pending[(c + 1) & 1]) {
+      cudaStreamWaitEvent(s, la->ev_rest[(c + 1) & 1], 0);  // update of step c - 1
+      pending[(c + 1) & 1] = false;
+    }
+    k_chol_step<<<c < 0 ? 1 : nblk - 1 - c, 256, kCholSmem, s>>>(A, n, n, c, work, d_info);
     ++launches;
-    const int rest = n - j0 - nb;
-    if (rest <= 0) continue;
-    k_panel_inplace<<<(rest + NB - 1) / NB, 256, 2 * kTileSmem, s>>>(A, n, j0, nb, rest, Db);
-    ++launches;
-    double* P = A + (j0 + nb) + static_cast<long long>(n) * j0;
-    double* A22 = A + (j0 + nb) + static_cast<long long>(n) * (j0 + nb);
+    if (c < 0) continue;
+    const int j0 = (c + 2) * NB, rest = n - j0;
+    if (rest <= NB) continue;  // nothing beyond the diagonal tile of the next steps
+    const double* P = A + j0 + static_cast<long long>(n) * (c * NB);
+    double* C = A + j0 + static_cast<long long>(n) * j0;
     if (!la) {
-      launches += syrk_update(rest, rest, nb, P, n, A22, n, s);
+      launches += syrk_update(rest, NB, P, n, C, n, s);
       continue;
     }
-    const int nb1 = std::min(NB, rest), rest2 = rest - nb1;
     cudaEventRecord(la->ev_panel, s);
-    // the previous step's remainder also updated this next block column
-    if (rest_pending) cudaStreamWaitEvent(s, la->ev_rest, 0);
-    launches += syrk_update(rest, nb1, nb, P, n, A22, n, s);
-    rest_pending = rest2 > 0;
-    if (rest_pending) {
-      cudaStreamWaitEvent(la->aux, la->ev_panel, 0);
-      launches += syrk_update(rest2, rest2, nb, P + nb1, n, A22 + nb1 + static_cast<long long>(n) * nb1, n,
-                              la->aux);
-      cudaEventRecord(la->ev_rest, la->aux);
-    }
+    cudaStreamWaitEvent(la->aux, la->ev_panel, 0);
+    launches += syrk_update(rest, NB, P, n, C, n, la->aux);
+    cudaEventRecord(la->ev_rest[c & 1], la->aux);
+    pending[c & 1] = true;
   }
-  if (rest_pending) cudaStreamWaitEvent(s, la->ev_rest, 0);
+  for (int p = 0; p < 2; ++p)
+    if (pending[p]) cudaStreamWaitEvent(s, la->ev_rest[p], 0);
   return launches;
 }
 

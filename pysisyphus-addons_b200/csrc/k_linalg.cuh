@@ -14,13 +14,12 @@ int gemm(bool ta, bool tb, int m, int n, int k, double alpha, const double* A, l
 // Doubles of scratch cholesky_lower needs for an n x n matrix (the inverted
 // 64 x 64 diagonal blocks, kept for trsm_lower_left).
 size_t linalg_workspace_doubles(int n);
-// Second stream of the Cholesky factorization: with it, the trailing update
-// beyond the next block column runs there while the next diagonal block is
-// factorized on the main stream (one step of lookahead). The events order the
-// two streams; all three are owned by the caller.
+// Second stream of the Cholesky factorization: with it, the trailing update of
+// a step runs there while the next step (panel and diagonal block) runs on the
+// main stream. The events order the two streams; all are owned by the caller.
 struct CholLookahead {
   cudaStream_t aux = nullptr;
-  cudaEvent_t ev_panel = nullptr, ev_rest = nullptr;
+  cudaEvent_t ev_panel = nullptr, ev_rest[2] = {};
 };
 // In place: the lower triangle of A (n x n, lda = n) becomes L with A = L L^T
 // (dpotrf); work receives the inverses of L's diagonal blocks. *d_info

@@ -512,7 +512,7 @@ int current_ctx(Ctx** out, DeviceTables* dt) {
       CholLookahead& la = i < Ctx::kNs3c ? c->la_met[i] : c->la2;
       PA_CUDA(cudaStreamCreateWithPriority(&la.aux, cudaStreamNonBlocking, prio_met));
       PA_CUDA(cudaEventCreateWithFlags(&la.ev_panel, cudaEventDisableTiming));
-      PA_CUDA(cudaEventCreateWithFlags(&la.ev_rest, cudaEventDisableTiming));
+      for (auto& e : la.ev_rest) PA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     PA_CUDA(cudaEventCreate(&c->m0));
     PA_CUDA(cudaEventCreate(&c->m1));
