@@ -48,16 +48,20 @@ __device__ __forceinline__ void cp_async16_ld(double* smem_dst, const double* gm
 // square root (the pivot's root follows from it and one Newton correction), per
 // 16-column sub-block
 //  * warp 0 factors the 16 x 16 diagonal sub-block (lane r holds row r, pivots
-//    and L(j, k) move by shuffles);
+//    and L(j, k) move by shuffles; ~345 cycles a pivot, and 490 with two columns
+//    per link through the 2 x 2 determinant: more dependent FP64 operations);
 //  * one thread per row below solves x L11^T = a in registers;
-//  * all threads update the trailing lower triangle.
+//  * the trailing lower triangle is updated on the FP64 tensor cores.
 // Inverse: four warps invert the diagonal sub-blocks (lane c holds column c,
 // right-looking, so a row's updates are independent), then the off-diagonal
-// blocks follow by doubling: X_21 = -X_22 (L_21 X_11) at 16 and at 32 columns.
+// blocks follow by doubling: X_21 = -X_22 (L_21 X_11) at 16 and at 32 columns,
+// on the FP64 tensor cores as well.
 constexpr int SB = 16;
 __device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X)[NB + 1], double (*T)[NB + 1],
                                                  double* invd, int nb, int pivot0, int* info) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t4 = lane & 3;
+  for (int idx = tid; idx < NB * NB; idx += 256) X[idx >> 6][idx & (NB - 1)] = 0.0;
   for (int k0 = 0; k0 < NB; k0 += SB) {
     if (warp == 0) {
       // lanes 16..31 repeat lanes 0..15 (they only feed the shuffles)
@@ -110,25 +114,33 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X
       for (int j = 0; j < SB; ++j) S[pr][k0 + j] = v[j];
     }
     __syncthreads();
-    // trailing lower triangle: S[r][c] -= sum_k S[r][k] S[c][k], k in the
-    // sub-block; a thread per entry of each 16 x 16 tile
-    const int ty = tid >> 4, tx = tid & 15;
-    for (int r0 = k0 + SB; r0 < NB; r0 += SB)
-      for (int c0 = k0 + SB; c0 <= r0; c0 += SB) {
-        const int rr = r0 + ty, cc = c0 + tx;
-        if (cc > rr) continue;
-        double v0 = 0.0, v1 = 0.0;
+    // trailing lower triangle: S -= P P^T of the sub-block's columns P, one 8 x 8
+    // tile per warp and turn
+    const int m8 = (NB - k0 - SB) / 8, tiles = m8 * (m8 + 1) / 2;  // 8-row tiles, at most 21
+    int tr[3], tc[3];
+    double d[3][2];
 #pragma unroll
-        for (int k = 0; k < SB; k += 2) {
-          v0 = fma(S[rr][k0 + k], S[cc][k0 + k], v0);
-          v1 = fma(S[rr][k0 + k + 1], S[cc][k0 + k + 1], v1);
-        }
-        S[rr][cc] -= v0 + v1;
+    for (int q = 0; q < 3; ++q) {
+      const int t = warp + 8 * q;
+      int bi = 0;
+      while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
+      tr[q] = k0 + SB + 8 * bi + g;
+      tc[q] = k0 + SB + 8 * (t - bi * (bi + 1) / 2);
+      d[q][0] = d[q][1] = 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < SB; k += 4)
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (warp + 8 * q < tiles) dmma_m8n8k4(d[q][0], d[q][1], S[tr[q]][k0 + k + t4], S[tc[q] + g][k0 + k + t4]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (warp + 8 * q < tiles) {
+        S[tr[q]][tc[q] + 2 * t4] -= d[q][0];
+        S[tr[q]][tc[q] + 2 * t4 + 1] -= d[q][1];
       }
     __syncthreads();
   }
-  for (int idx = tid; idx < NB * NB; idx += 256) X[idx >> 6][idx & (NB - 1)] = 0.0;
-  __syncthreads();
   if (warp < NB / SB) {
     const int o = warp * SB, c = lane & (SB - 1);
     double x[SB];
@@ -148,37 +160,42 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X
     }
   }
   __syncthreads();
-  // doubling: blocks of w columns, T = L_21 X_11 (X_11 lower triangular), then
-  // X_21 = -X_22 T; every sum in two interleaved halves
+  // doubling: blocks of w columns, T = L_21 X_11, then X_21 = -X_22 T, 8 x 8
+  // tiles over the warps
   auto level = [&](auto wc) {
     constexpr int w = decltype(wc)::value;
-    constexpr int npair = NB / (2 * w), per = npair * w * w / 256;
+    constexpr int turns = (NB / (2 * w)) * (w / 8) * (w / 8) / 8;
+    int o[turns], i[turns], j[turns];
 #pragma unroll
-    for (int q = 0; q < per; ++q) {
-      const int e = tid + 256 * q;
-      const int pairi = e / (w * w), i = (e / w) % w, j = e % w, o = pairi * 2 * w;
-      double v0 = 0.0, v1 = 0.0;
-#pragma unroll
-      for (int k = 0; k < w; k += 2) {
-        v0 = fma(S[o + w + i][o + k], X[o + k][o + j], v0);
-        v1 = fma(S[o + w + i][o + k + 1], X[o + k + 1][o + j], v1);
-      }
-      T[o + w + i][j] = v0 + v1;
+    for (int t = 0; t < turns; ++t) {
+      const int id = warp + 8 * t;
+      o[t] = id / ((w / 8) * (w / 8)) * 2 * w;
+      i[t] = o[t] + w + id / (w / 8) % (w / 8) * 8 + g;
+      j[t] = id % (w / 8) * 8;
     }
-    __syncthreads();
 #pragma unroll
-    for (int q = 0; q < per; ++q) {
-      const int e = tid + 256 * q;
-      const int pairi = e / (w * w), i = (e / w) % w, j = e % w, o = pairi * 2 * w;
-      double v0 = 0.0, v1 = 0.0;
+    for (int half = 0; half < 2; ++half) {
+      double d[turns][2][2] = {};  // per tile two chains of products
 #pragma unroll
-      for (int k = 0; k < w; k += 2) {
-        v0 = fma(X[o + w + i][o + w + k], T[o + w + k][j], v0);
-        v1 = fma(X[o + w + i][o + w + k + 1], T[o + w + k + 1][j], v1);
-      }
-      X[o + w + i][o + j] = -(v0 + v1);
+      for (int k = 0; k < w; k += 4)
+#pragma unroll
+        for (int t = 0; t < turns; ++t) {
+          const double a = half == 0 ? S[i[t]][o[t] + k + t4] : X[i[t]][o[t] + w + k + t4];
+          const double b = half == 0 ? X[o[t] + k + t4][o[t] + j[t] + g] : T[o[t] + w + k + t4][j[t] + g];
+          dmma_m8n8k4(d[t][k / 4 & 1][0], d[t][k / 4 & 1][1], a, b);
+        }
+#pragma unroll
+      for (int t = 0; t < turns; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double v = d[t][0][e] + d[t][1][e];
+          if (half == 0)
+            T[i[t]][j[t] + 2 * t4 + e] = v;
+          else
+            X[i[t]][o[t] + j[t] + 2 * t4 + e] = -v;
+        }
+      __syncthreads();
     }
-    __syncthreads();
   };
   level(std::integral_constant<int, SB>{});
   level(std::integral_constant<int, 2 * SB>{});
@@ -260,6 +277,18 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
         const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
         cv[mt][nt][e] = (c >= 0 && r < nr) ? Ac[r + lda * j] : 0.0;
       }
+  // block 0: its entries of the next diagonal block (rows past n: identity)
+  double* Ai = A + r0 + lda * static_cast<long long>(r0);
+  double dv[2][4][2];
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
+        dv[mt][nt][e] = (diag && r < nr && j <= r) ? Ai[r + lda * j] : (r == j ? 1.0 : 0.0);
+      }
   double acc[2][4][2];
   auto clear = [&] {
 #pragma unroll
@@ -309,17 +338,7 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
         for (int e = 0; e < 2; ++e)
           Ds[(wn + 8 * nt + 2 * t4 + e) * kPanLd + wm + 8 * mt + g] = acc[mt][nt][e];
   }
-  // the next diagonal block (rows past n: identity)
-  double* Ai = A + r0 + lda * static_cast<long long>(r0);
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
-        cv[mt][nt][e] = (r < nr && j <= r) ? Ai[r + lda * j] : (r == j ? 1.0 : 0.0);
-      }
+  // the next diagonal block
   __syncthreads();
   for (int term = 0; term < 2; ++term) {  // columns c - 1, then c
     if (c < 1 - term) continue;
@@ -330,7 +349,7 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) cv[mt][nt][e] -= acc[mt][nt][e];
+        for (int e = 0; e < 2; ++e) dv[mt][nt][e] -= acc[mt][nt][e];
   }
   double(*S)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(Bs);
   double(*X)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(As);
@@ -342,7 +361,7 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int r = wm + 8 * mt + g, j = wn + 8 * nt + 2 * t4 + e;
-        S[r][j] = j <= r ? cv[mt][nt][e] : 0.0;
+        S[r][j] = j <= r ? dv[mt][nt][e] : 0.0;
       }
   __syncthreads();  // As and Ds are free as well
   factor_invert_64(S, X, T, invd, nr, r0, info);
@@ -354,112 +373,179 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
   }
 }
 
-// Super-step of the blocked forward substitution B := L^-1 B (right-looking)
-// over the diagonal blocks k0 .. k0 + ns - 1 (ns <= kTrsmSuper). Block
-// (it, jt), it = k0.., jt over 16-column tiles of B, first solves the
-// super-step's blocks itself, in the order of the one-block-per-launch scheme:
-// for j = 0 .. ns-1, B_(k0+j) -= L_(k0+j, k0+l) X_l for l < j, then
-// X_j = Dinv_(k0+j) B_(k0+j). Every product is sum_p M[r][p] X[p][c] with p
-// ascending and each update one subtraction, so the results are those of one
-// launch per diagonal block, in a quarter of the launches. Blocks with it in
-// the super-step store X_(it-k0) in C; the others update
-// B_it -= L_(it, k0+j) X_j for j = 0 .. ns-1 (B itself is only written by
-// these, and B_(k0..) is read before any block of this launch writes). Thread
-// (r, g) = (tid % 64, tid / 64) owns row r, columns 4 g .. 4 g + 3 of the tile.
-constexpr int kTrsmCols = 16;
-constexpr int kTrsmSuper = 4;
-constexpr size_t kTrsmSmem = sizeof(double) * (NB * (NB + 1) + kTrsmSuper * NB * (kTrsmCols + 1));
-__global__ void __launch_bounds__(256) k_trsm_super(const double* __restrict__ L, long long lda, int n,
-                                                    int k0, int ns, const double* __restrict__ dinv,
-                                                    const double* B, long long ldb, int nrhs, double* Bw,
-                                                    double* C, long long ldc) {
-  extern __shared__ double tsm[];
-  double(*M)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(tsm);  // Dinv or an L block   [i][p]
-  double(*Xs)[NB][kTrsmCols + 1] =
-      reinterpret_cast<double(*)[NB][kTrsmCols + 1]>(tsm + NB * (NB + 1));  // X_j     [j][p][c]
-  const int tid = threadIdx.x, r = tid & (NB - 1), g = tid >> 6;
-  const int it = k0 + blockIdx.x, c0 = blockIdx.y * kTrsmCols;
-  auto load_M = [&](const double* src, long long ld, int rows, int cols) {
-    __syncthreads();  // every thread is done with M
+// One launch of the blocked forward substitution X = L^-1 B over R 64-row
+// blocks of L from row k0 (a super-step). Two kinds of blocks, 8 warps each:
+//  * the first nsolve blocks, one per 8 columns of B: apply X of the previous
+//    super-step to the rows of this one, then solve them 64 at a time with the
+//    inverted diagonal blocks, X_j = Dinv_j (B_j - sum_(l < j) L_jl X_l);
+//  * the others, one per 64 rows below and 8 NT columns: B -= L X of the previous
+//    super-step.
+// So a super-step is one launch, its serial part overlaps the update below it,
+// and nothing is solved twice. Products on the FP64 tensor cores (mma.sync
+// m8n8k4): warp w owns rows 8 w.. of a 64-row block and reads its L fragments
+// straight from global memory (8 rows = 64 contiguous bytes), ahead of the
+// barriers that guard X, which is shared through shared memory.
+//
+// Bound: for few columns the solving blocks' chain of loads and barriers, so
+// R = 2 with every fragment of a step in registers (one block per SM); for many
+// the FP64 tensor pipe, so R = 4 (half the passes over B, two blocks per SM).
+constexpr int kTrsmFew = 192;  // densities of up to 19 states
+constexpr int kTrsmLdx = 12;  // 4 or 12 (mod 16): conflict-free fragment loads
+constexpr size_t trsm_smem(int nt, int nblk) {
+  return sizeof(double) * std::max(nblk * NB * (8 * nt + 4), nblk * NB * kTrsmLdx + 2 * NB * kTrsmLdx);
+}
+
+template <int NT, int R>
+__global__ void __launch_bounds__(256, R == 2 ? 1 : 2) k_trsm_step(const double* __restrict__ L, long long lda, int n,
+                                                                   int k0, const double* __restrict__ dinv, double* B,
+                                                                   long long ldb, int nrhs, double* C, long long ldc,
+                                                                   int nsolve) {
+  extern __shared__ __align__(16) double tsm[];
+  constexpr int kRows = R * NB, kQ = NB / 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int kp = k0 - kRows;  // rows of the previous super-step (all below n)
+  if (static_cast<int>(blockIdx.x) < nsolve) {
+    double* Xp = tsm;                        // [k][col] X of the previous super-step
+    double* T = Xp + kRows * kTrsmLdx;       // [row][col] right-hand side of one block
+    double* Xn = T + NB * kTrsmLdx;          // [row][col] its solution
+    const int c0 = blockIdx.x * 8, row0 = k0 + 8 * warp + g;
+    double bv[R][2], acc[R][2];
 #pragma unroll
-    for (int idx = tid; idx < NB * NB; idx += 256) {
-      const int i = idx & (NB - 1), q = idx >> 6;
-      M[i][q] = (i < rows && q < cols) ? src[i + ld * q] : 0.0;
-    }
-    __syncthreads();
-  };
-  // the super-step's solutions X_0 .. X_(ns-1), kept in shared memory
-  for (int j = 0; j < ns; ++j) {
-    const int rj = (k0 + j) * NB, nbj = min(NB, n - rj);
-    double t[4];
+    for (int j = 0; j < R; ++j)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int col = c0 + 4 * g + c;
-      t[c] = (r < nbj && col < nrhs) ? B[(rj + r) + ldb * col] : 0.0;
-    }
-    for (int l = 0; l < j; ++l) {
-      const int rl = (k0 + l) * NB, nbl = min(NB, n - rl);
-      load_M(L + rj + lda * rl, lda, nbj, nbl);
-      double upd[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-      for (int p = 0; p < NB; ++p) {
-        const double m = M[r][p];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) upd[c] = fma(m, Xs[l][p][4 * g + c], upd[c]);
+      for (int e = 0; e < 2; ++e) {
+        const int row = row0 + NB * j, col = c0 + 2 * t4 + e;
+        bv[j][e] = (row < n && col < nrhs) ? B[row + ldb * col] : 0.0;
+        acc[j][e] = 0.0;
       }
+    if (kp >= 0) {
+      // fragments of 64 columns of L at a time, the next ones in flight while
+      // the current ones are multiplied
+      const double* l = L + row0 + lda * (kp + t4);
+      double a[2][R][kQ];
+      auto fetch = [&](int h, double (&f)[R][kQ]) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) t[c] -= upd[c];
-    }
-    // X_j = Dinv_j t: t goes through shared memory (row r of the tile)
+        for (int j = 0; j < R; ++j)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) Xs[j][r][4 * g + c] = (r < nbj) ? t[c] : 0.0;
-    load_M(dinv + static_cast<size_t>(k0 + j) * NB * NB, NB, NB, NB);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+          for (int q = 0; q < kQ; ++q) f[j][q] = row0 + NB * j < n ? l[NB * j + lda * (NB * h + 4 * q)] : 0.0;
+      };
+      if constexpr (R == 2) fetch(0, a[0]);
+      for (int idx = tid; idx < kRows * 8; idx += 256) {
+        const int r = idx & (kRows - 1), c = idx / kRows;
+        Xp[r * kTrsmLdx + c] = c0 + c < nrhs ? C[(kp + r) + ldc * (c0 + c)] : 0.0;
+      }
+      __syncthreads();
+      if constexpr (R == 2) {
+        double part[R][4][2] = {};  // independent chains of products
+#pragma unroll
+        for (int h = 0; h < R; ++h) {
+          if (h + 1 < R) fetch(h + 1, a[(h + 1) & 1]);
+#pragma unroll
+          for (int q = 0; q < kQ; ++q) {
+            const double b = Xp[(NB * h + 4 * q + t4) * kTrsmLdx + g];
+#pragma unroll
+            for (int j = 0; j < R; ++j) dmma_m8n8k4(part[j][q & 3][0], part[j][q & 3][1], a[h & 1][j][q], b);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) acc[j][e] = (part[j][0][e] + part[j][1][e]) + (part[j][2][e] + part[j][3][e]);
+      } else {
 #pragma unroll 8
-    for (int p = 0; p < NB; ++p) {
-      const double m = M[r][p];
+        for (int k = 0; k < kRows; k += 4) {
+          const double b = Xp[(k + t4) * kTrsmLdx + g];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[c] = fma(m, Xs[j][p][4 * g + c], acc[c]);
+          for (int j = 0; j < R; ++j)
+            dmma_m8n8k4(acc[j][0], acc[j][1], row0 + NB * j < n ? l[NB * j + lda * k] : 0.0, b);
+        }
+      }
     }
-    __syncthreads();  // every thread has read Xs[j] as B_j
 #pragma unroll
-    for (int c = 0; c < 4; ++c) Xs[j][r][4 * g + c] = acc[c];
-  }
-  if (it < k0 + ns) {
-    __syncthreads();
-    const int j = it - k0, rj = it * NB, nbj = min(NB, n - rj);
+    for (int j = 0; j < R; ++j) {
+      if (k0 + NB * j >= n) break;
+      const int row = row0 + NB * j;
+      const bool rowok = row < n;
+      // Dinv_j and the tile of L that the next block waits for, before the barrier
+      const double* dj = dinv + static_cast<size_t>(k0 / NB + j) * NB * NB + 8 * warp + g;
+      const double* l = L + row0 + lda * (k0 + NB * j + t4);
+      double da[kQ], ln[kQ];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int col = c0 + 4 * g + c;
-      if (r < nbj && col < nrhs) C[(rj + r) + ldc * col] = Xs[j][r][4 * g + c];
+      for (int q = 0; q < kQ; ++q) da[q] = 4 * q < 8 * (warp + 1) ? dj[NB * (4 * q + t4)] : 0.0;
+      if (j + 1 < R)
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) ln[q] = row + NB < n ? l[NB * (j + 1) + lda * (4 * q)] : 0.0;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) T[(8 * warp + g) * kTrsmLdx + 2 * t4 + e] = rowok ? bv[j][e] - acc[j][e] : 0.0;
+      __syncthreads();
+      double x[4][2] = {};  // independent chains of products
+#pragma unroll
+      for (int q = 0; q < kQ; ++q)  // columns past the warp's rows of Dinv are zero
+        if (4 * q < 8 * (warp + 1)) dmma_m8n8k4(x[q & 3][0], x[q & 3][1], da[q], T[(4 * q + t4) * kTrsmLdx + g]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const double v = (x[0][e] + x[1][e]) + (x[2][e] + x[3][e]);
+        const int col = c0 + 2 * t4 + e;
+        Xn[(8 * warp + g) * kTrsmLdx + 2 * t4 + e] = v;
+        if (rowok && col < nrhs) C[row + ldc * col] = v;
+      }
+      if (j + 1 >= R) break;
+      __syncthreads();
+      double y[4][2] = {};
+#pragma unroll
+      for (int q = 0; q < kQ; ++q)
+        dmma_m8n8k4(y[q & 3][0], y[q & 3][1], ln[q], Xn[(4 * q + t4) * kTrsmLdx + g]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) acc[(j + 1) % R][e] += (y[0][e] + y[1][e]) + (y[2][e] + y[3][e]);
+      if constexpr (R > 2) {
+#pragma unroll 4
+        for (int k = 0; k < NB; k += 4) {
+          const double b = Xn[(k + t4) * kTrsmLdx + g];
+#pragma unroll
+          for (int q = 2; q < R; ++q) {
+            if (q <= j + 1) continue;
+            dmma_m8n8k4(acc[q][0], acc[q][1], row0 + NB * q < n ? l[NB * q + lda * k] : 0.0, b);
+          }
+        }
+      }
     }
     return;
   }
-  const int ri = it * NB, nbi = min(NB, n - ri);
-  double bv[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int col = c0 + 4 * g + c;
-    bv[c] = (r < nbi && col < nrhs) ? B[(ri + r) + ldb * col] : 0.0;
+  constexpr int kLd = 8 * NT + 4;
+  double* Xs = tsm;  // [k][col]
+  const int r1 = k0 + kRows, nrow = (n - r1 + NB - 1) / NB;
+  const int blk = blockIdx.x - nsolve, c0 = (blk / nrow) * 8 * NT;
+  const int row = r1 + (blk % nrow) * NB + 8 * warp + g;
+  const bool rowok = row < n;
+  for (int idx = tid; idx < kRows * 8 * NT; idx += 256) {
+    const int r = idx & (kRows - 1), c = idx / kRows;
+    Xs[r * kLd + c] = c0 + c < nrhs ? C[(kp + r) + ldc * (c0 + c)] : 0.0;
   }
-  for (int j = 0; j < ns; ++j) {
-    const int rj = (k0 + j) * NB, nbj = min(NB, n - rj);
-    load_M(L + ri + lda * rj, lda, nbi, nbj);
-    double upd[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-    for (int p = 0; p < NB; ++p) {
-      const double m = M[r][p];
+  double bv[NT][2], acc[NT][2];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) upd[c] = fma(m, Xs[j][p][4 * g + c], upd[c]);
+  for (int q = 0; q < NT; ++q)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int col = c0 + 8 * q + 2 * t4 + e;
+      bv[q][e] = (rowok && col < nrhs) ? B[row + ldb * col] : 0.0;
+      acc[q][e] = 0.0;
     }
+  __syncthreads();
+  const double* l = L + row + lda * (kp + t4);
+#pragma unroll 16
+  for (int k = 0; k < kRows; k += 4) {
+    const double a = rowok ? l[lda * k] : 0.0;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) bv[c] -= upd[c];
+    for (int q = 0; q < NT; ++q) dmma_m8n8k4(acc[q][0], acc[q][1], a, Xs[(k + t4) * kLd + 8 * q + g]);
   }
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int col = c0 + 4 * g + c;
-    if (r < nbi && col < nrhs) Bw[(ri + r) + ldb * col] = bv[c];
-  }
+  for (int q = 0; q < NT; ++q)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int col = c0 + 8 * q + 2 * t4 + e;
+      if (rowok && col < nrhs) B[row + ldb * col] = bv[q][e] - acc[q][e];
+    }
 }
 
 // C[m x n] := beta C + alpha op(A) op(B); op(A) is m x k, op(B) is k x n.
@@ -773,17 +859,32 @@ int cholesky_lower(double* A, int n, int* d_info, double* work, cudaStream_t s,
   return launches;
 }
 
+namespace {
+
+template <int NT, int R>
+int trsm_launches(const double* L, int n, const double* dinv, double* B, long long ldb, int nrhs, double* C,
+                  long long ldc, cudaStream_t s) {
+  constexpr int kRows = R * NB;
+  const size_t smem = trsm_smem(NT, R);
+  cudaFuncSetAttribute(k_trsm_step<NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const int nsolve = (nrhs + 7) / 8, ct = (nrhs + 8 * NT - 1) / (8 * NT);
+  int launches = 0;
+  for (int k0 = 0; k0 < n; k0 += kRows, ++launches) {
+    const int below = k0 > 0 ? std::max(0, n - k0 - kRows) : 0;
+    const long long blocks = nsolve + static_cast<long long>((below + NB - 1) / NB) * ct;
+    k_trsm_step<NT, R><<<static_cast<unsigned>(blocks), 256, smem, s>>>(L, n, n, k0, dinv, B, ldb, nrhs, C, ldc, nsolve);
+  }
+  return launches;
+}
+
+}  // namespace
+
 int trsm_lower_left(const double* L, int n, const double* dinv, double* B, long long ldb, int nrhs,
                     double* C, long long ldc, cudaStream_t s) {
   if (n <= 0 || nrhs <= 0) return 0;
-  cudaFuncSetAttribute(k_trsm_super, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTrsmSmem));
-  const int nblk = (n + NB - 1) / NB, ct = (nrhs + kTrsmCols - 1) / kTrsmCols;
-  int launches = 0;
-  for (int k0 = 0; k0 < nblk; k0 += kTrsmSuper, ++launches) {
-    const int ns = std::min(kTrsmSuper, nblk - k0);
-    k_trsm_super<<<dim3(nblk - k0, ct), 256, kTrsmSmem, s>>>(L, n, n, k0, ns, dinv, B, ldb, nrhs, B, C, ldc);
-  }
-  return launches;
+  if (nrhs <= 40) return trsm_launches<5, 2>(L, n, dinv, B, ldb, nrhs, C, ldc, s);
+  if (nrhs <= kTrsmFew) return trsm_launches<4, 2>(L, n, dinv, B, ldb, nrhs, C, ldc, s);
+  return trsm_launches<4, 4>(L, n, dinv, B, ldb, nrhs, C, ldc, s);
 }
 
 int add_diagonal(double* A, int n, double shift, cudaStream_t s) {
