@@ -326,6 +326,10 @@ int pa_int3c2e_estimates(pa_basis orbital, pa_basis aux, long long cap, double* 
 int f_eval_densities(int nshells, int ndata, const int* bas_centers, const int* bas_spec,
                      const double* bas_data, int npoints, const double* grid3d, int ndens, int nbfs,
                      const double* densities, double* grid_densities, int blk_size, double thresh);
+/* The same with the densities in `layout` (PA_LAYOUT_C: density, row, column). */
+int pa_eval_densities(int nshells, int ndata, const int* bas_centers, const int* bas_spec,
+                      const double* bas_data, int npoints, const double* grid3d, int ndens, int nbfs,
+                      const double* densities, int layout, double* grid_densities, int blk_size, double thresh);
 /* Density of the primitive pairs with exponent sum below `sw` on grid points
  * (replaces gdma/prim_dens.f90:100-259, f_eval_prim_density, same arguments):
  * ls_inds(2, nprims) = (L, 0-based Cartesian start), primdata(5, nprims) =
@@ -334,6 +338,9 @@ int f_eval_densities(int nshells, int ndata, const int* bas_centers, const int* 
  * the 15 components; these are all 15). Host buffers; synchronous. */
 int f_eval_prim_density(int nprims, int npoints, int nbfs, const int* ls_inds, const double* primdata,
                         const double* coords3d, const double* P, double sw, double* rho);
+/* The same with P in `layout`. */
+int pa_eval_prim_density(int nprims, int npoints, int nbfs, const int* ls_inds, const double* primdata,
+                         const double* coords3d, const double* P, int layout, double sw, double* rho);
 
 /* The metric half of contract_coulomb_densities_2d / _4d on device buffers
  * (common/linalg.f90:60-82 inv_chol, diabatization/intor.f90:198 dtrmm and

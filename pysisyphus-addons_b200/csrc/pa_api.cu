@@ -2128,8 +2128,11 @@ int pa_get_precision(void) {
 
 int pa_basis_cache_clear(void) {
   pa::BasisCache& cache = pa::basis_cache();
-  std::lock_guard<std::mutex> lk(cache.mu);
-  cache.entries.clear();
+  {
+    std::lock_guard<std::mutex> lk(cache.mu);
+    cache.entries.clear();
+  }
+  release_grid_pools();
   return PA_OK;
 }
 

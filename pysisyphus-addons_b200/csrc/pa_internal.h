@@ -152,4 +152,7 @@ int launch_schwarz_aux(const DevBasis& X, const DeviceTables& dt, int boys_mode,
 int launch_metric(const DevBasis& X, const DeviceTables& dt, int boys_mode, double* M,
                   cudaStream_t s);
 
+// Gives back the memory and idle streams the grid densities keep between calls.
+void release_grid_pools();
+
 }  // namespace pa

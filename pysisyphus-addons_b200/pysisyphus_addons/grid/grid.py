@@ -1,9 +1,9 @@
 """Densities on grid points (reference: pysisyphus_addons/grid/grid.py:1-22 and
 grid/_grid.pyx:35-75; Fortran driver grid/grid.f90:110-286).
 
-The functions call the reference-compatible C-ABI entry point f_eval_densities
-of libpa_b200.so with host arrays, as the reference's Cython module does, and
-return F-ordered numpy arrays. The computation runs on the current CUDA device.
+The functions call pa_eval_densities of libpa_b200.so (the reference-compatible
+f_eval_densities with a layout argument) with host arrays and return F-ordered
+numpy arrays. The computation runs on the current CUDA device.
 """
 
 import numpy as np
@@ -29,12 +29,16 @@ def eval_densities(shells, grid3d, densities, blk_size=100, thresh=1e-8):
     G = np.asfortranarray(np.asarray(grid3d, dtype=np.float64).T)  # (3, npoints)
     if G.ndim != 2 or G.shape[0] != 3:
         raise ValueError("grid3d must have shape (npoints, 3)")
-    D = np.asfortranarray(densities, dtype=np.float64)
+    D = np.asarray(densities, dtype=np.float64)
+    # either order is read in place; anything else is copied
+    layout = nat.PA_LAYOUT_C if D.flags.c_contiguous else nat.PA_LAYOUT_FORTRAN
+    if layout == nat.PA_LAYOUT_FORTRAN:
+        D = np.asfortranarray(D)
     if D.ndim != 3 or D.shape[1] != D.shape[2]:
         raise ValueError("densities must have shape (ndens, nbfs, nbfs)")
     ndens, nbfs = D.shape[0], D.shape[1]
     npoints = G.shape[1]
     out = np.zeros((ndens, npoints), dtype=np.float64, order="F")
-    nat.check(nat.load().f_eval_densities(*b, npoints, nat.ptr(G), ndens, nbfs, nat.ptr(D), nat.ptr(out),
-                                          int(blk_size), float(thresh)))
+    nat.check(nat.load().pa_eval_densities(*b, npoints, nat.ptr(G), ndens, nbfs, nat.ptr(D), layout, nat.ptr(out),
+                                           int(blk_size), float(thresh)))
     return out
