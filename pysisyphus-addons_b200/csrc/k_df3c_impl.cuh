@@ -323,13 +323,80 @@ __device__ __forceinline__ void x_triplet_thread(const Df3cArgs& a, double p, do
   }
 }
 
+// Recurrence for R by a team (L > 5). The direction rule (x before y before z)
+// makes every R_tuv with t > 0 depend on entries of its own (u, v) column alone,
+//   R^n_(t+1)uv = X R^(n+1)_tuv + t R^(n+1)_(t-1)uv,
+// so only the plane t = 0 is built level by level through shared memory (C(L+3, 3)
+// entries over all levels instead of C(L+4, 4): 165 of 495 for L = 8), all of its
+// levels kept; then each lane takes whole columns, R^n_0uv, n = 0 .. L - u - v, to
+// R^0_tuv, t = 0 .. L - u - v, in registers. The same operations per entry as the
+// level-by-level form (bit for bit), a third of its shared-memory accesses.
+// Plane entry (u, v) of degree d = u + v has index d (d + 1) / 2 + v, at every
+// level; R^0_tuv is then component ncum(d + t - 1) + that index.
+__host__ __device__ constexpr int plane_off(int L, int n) { return ncum(L) - ncum(L - n); }  // level n's first entry
+__host__ __device__ constexpr int plane_degree(int i) {
+  int d = 0;
+  while ((d + 1) * (d + 2) / 2 <= i) ++d;
+  return d;
+}
+
+// Plane descriptor: s1 | s2 << 7 | c << 14 | z << 18 | degree << 19, so that
+// R(i) = (z ? Z : Y) R'(s1) + c R'(s2).
+template <int L>
+__device__ __forceinline__ void fill_team_tables(uchar4* txyz, int* pdesc, const DeviceTables& dt, int tid) {
+  static_assert(ncart(L) <= 128 && L < 16, "descriptor fields");
+  for (int i = tid; i < ncum(L); i += kThreads) txyz[i] = *reinterpret_cast<const uchar4*>(dt.idx->xyz[i]);
+  for (int i = tid; i < ncart(L); i += kThreads) {
+    const int d = plane_degree(i), v = i - d * (d + 1) / 2, u = d - v;
+    const int e = u > 0 ? u : v;                // exponent of the recurrence's direction
+    const int v1 = u > 0 ? v : v - 1, v2 = u > 0 ? v : v - 2;
+    const int s1 = d > 0 ? (d - 1) * d / 2 + v1 : 0, s2 = e > 1 ? (d - 2) * (d - 1) / 2 + v2 : 0;
+    pdesc[i] = s1 | s2 << 7 | (e > 1 ? e - 1 : 0) << 14 | (u > 0 ? 0 : 1) << 18 | d << 19;
+  }
+}
+
+// One column of degree d (at least L - M): plane points at its entry of level
+// 0, out at its component t = 0.
+template <int L, int M, class Real>
+__device__ __forceinline__ void hermite_column(Real X, const Real* plane, int d, Real* out) {
+  Real c[2][M + 1];
+#pragma unroll
+  for (int n = 0; n <= M; ++n) c[0][n] = n + d <= L ? plane[plane_off(L, n)] : static_cast<Real>(0);
+  *out = c[0][0];
+  int step = (d + 1) * (d + 2) / 2;
+#pragma unroll
+  for (int t = 1; t <= M; ++t) {
+#pragma unroll
+    for (int n = 0; n <= M - t; ++n) {
+      Real v = X * c[(t - 1) & 1][n + 1];
+      if (t > 1) v = fma(static_cast<Real>(t - 1), c[t & 1][n + 1], v);
+      c[t & 1][n] = v;
+    }
+    out += step;
+    step += d + t + 1;
+    if (d + t <= L) *out = c[t & 1][0];
+  }
+}
+
+template <int L, int TS, int IT, class Real>
+__device__ __forceinline__ void hermite_columns(Real X, const Real* plane, const int* pdesc, int tl, Real* R) {
+  constexpr int first = IT * TS;
+  if constexpr (first < ncart(L)) {
+    const int i = first + tl;
+    if (i < ncart(L)) {
+      const int d = pdesc[i] >> 19;
+      hermite_column<L, L - plane_degree(first), Real>(X, plane + i, d, R + ncum(d - 1) + i);
+    }
+    hermite_columns<L, TS, IT + 1, Real>(X, plane, pdesc, tl, R);
+  }
+}
+
 // X of one triplet by a team of TS threads (L > 5): orders of the Boys
-// function across lanes, R level by level in shared memory, X rows across the
-// lanes. Every thread of a warp (of a team, for teams larger than a warp)
-// calls this with the same Real (the caller makes the precision choice
-// uniform), so the team barriers pair up.
+// function across lanes, R as above, X rows across the lanes. Every thread of a
+// warp (of a team, for teams larger than a warp) calls this with the same Real
+// (the caller makes the precision choice uniform), so the team barriers pair up.
 template <int LAB, int LC, int TS, class Real>
-__device__ __forceinline__ void x_triplet_team(const Df3cArgs& a, const uchar4* txyz, const int* rdesc,
+__device__ __forceinline__ void x_triplet_team(const Df3cArgs& a, const uchar4* txyz, const int* pdesc,
                                                double* rbuf, int team, int tl, bool active, int np, int po,
                                                int maxprim, double p, double X, double Y, double Z,
                                                double* xrow, int mpad) {
@@ -337,8 +404,8 @@ __device__ __forceinline__ void x_triplet_team(const Df3cArgs& a, const uchar4* 
   constexpr int NR = ncum(L);
   constexpr int NH = ncum(LAB);
   Real* Rn = reinterpret_cast<Real*>(rbuf);
-  Real* b0 = Rn + 16;
-  Real* b1 = b0 + NR;
+  Real* b0 = Rn + 16;      // R^0
+  Real* plane = b0 + NR;   // R^n_0uv of every level
   const double RPC2 = X * X + Y * Y + Z * Z;
   const Real Xr = static_cast<Real>(X), Yr = static_cast<Real>(Y), Zr = static_cast<Real>(Z);
   for (int kp = 0; kp < maxprim; ++kp) {
@@ -357,39 +424,37 @@ __device__ __forceinline__ void x_triplet_team(const Df3cArgs& a, const uchar4* 
       }
     }
     team_sync<TS>(team);
-    // Hermite R, level by level. The loops have compile-time trip counts and
-    // are unrolled: the components of one level are independent, so their
+    // the plane, level by level. The loops have compile-time trip counts and
+    // are unrolled: the entries of one level are independent, so their
     // descriptor and operand loads are issued back to back instead of one
-    // dependent load chain per component.
-    {
-      Real* top = (L & 1) ? b1 : b0;
-      if (has && tl == 0) top[0] = Rn[L];
-      team_sync<TS>(team);
+    // dependent load chain per entry
+    if (has && tl == 0) plane[plane_off(L, L)] = Rn[L];
+    team_sync<TS>(team);
 #pragma unroll
-      for (int n = L - 1; n >= 0; --n) {
-        Real* dst = (n & 1) ? b1 : b0;
-        const Real* src = (n & 1) ? b0 : b1;
-        const int cnt = ncum(L - n);
+    for (int n = L - 1; n >= 0; --n) {
+      Real* dst = plane + plane_off(L, n);
+      const Real* src = plane + plane_off(L, n + 1);
+      const int cnt = ncart(L - n);
 #pragma unroll
-        for (int it = 0; it < (cnt + TS - 1) / TS; ++it) {
-          const int idx = tl + it * TS;
-          if (has && idx < cnt) {
-            Real v;
-            if (idx == 0) {
-              v = Rn[n];
-            } else {
-              const int dsc = rdesc[idx];
-              const int d = rdesc_d(dsc), c = rdesc_c(dsc);
-              const Real xd = d == 0 ? Xr : (d == 1 ? Yr : Zr);
-              v = xd * src[rdesc_s1(dsc)];
-              if (c) v = fma(static_cast<Real>(c), src[rdesc_s2(dsc)], v);
-            }
-            dst[idx] = v;
+      for (int it = 0; it < (cnt + TS - 1) / TS; ++it) {
+        const int idx = tl + it * TS;
+        if (has && idx < cnt) {
+          Real v;
+          if (idx == 0) {
+            v = Rn[n];
+          } else {
+            const int dsc = pdesc[idx];
+            const int c = (dsc >> 14) & 15;
+            v = ((dsc >> 18) & 1 ? Zr : Yr) * src[dsc & 127];
+            if (c) v = fma(static_cast<Real>(c), src[(dsc >> 7) & 127], v);
           }
+          dst[idx] = v;
         }
-        team_sync<TS>(team);
       }
+      team_sync<TS>(team);
     }
+    if (has) hermite_columns<L, TS, 0, Real>(Xr, plane, pdesc, tl, b0);
+    team_sync<TS>(team);
     // X rows: lanes over the Hermite components t of the bra, compile-time
     // solid-harmonic terms of the auxiliary shell (the first primitive stores)
 #pragma unroll
@@ -482,7 +547,6 @@ __device__ __forceinline__ void df3c_item(const Df3cArgs& a, int bx, int by, int
   for (int i = 0; i < tile_n; ++i) maxprim = max(maxprim, c_info[2 * i]);
   const double qc_max = tile_n > 0 ? c_C[0].w : 0.0;
   const double thr = a.thresh;
-  const IndexTables* it = a.dt.idx;
   // the units that can meet the tile form a prefix of the sorted class (the
   // staircase); the item takes chunk `by` of nby equal chunks of that prefix,
   // so every item of a tile has the same number of steps
@@ -579,12 +643,9 @@ __device__ __forceinline__ void df3c_item(const Df3cArgs& a, int bx, int by, int
     } else {
       // team index tables (shared memory copies of the decoded multi-indices)
       uchar4* txyz = reinterpret_cast<uchar4*>(Rteam + C::NTRIP * C::kTeamStride);
-      int* rdesc = reinterpret_cast<int*>(txyz + C::NR);
+      int* pdesc = reinterpret_cast<int*>(txyz + C::NR);
       if (u0 == ub) {
-        for (int i = tid; i < C::NR; i += kThreads) {
-          txyz[i] = *reinterpret_cast<const uchar4*>(it->xyz[i]);
-          rdesc[i] = a.dt.rdesc[i];
-        }
+        fill_team_tables<C::L>(txyz, pdesc, a.dt, tid);
         __syncthreads();
       }
       const int team = tid / C::TS, tl = tid - team * C::TS;
@@ -608,10 +669,10 @@ __device__ __forceinline__ void df3c_item(const Df3cArgs& a, int bx, int by, int
       const bool weak = !active || est < a.thr32;
       const bool f32 = __all_sync(0xffffffffu, weak) && __any_sync(0xffffffffu, active);
       if (f32)
-        x_triplet_team<LAB, LC, C::TS, float>(a, txyz, rdesc, rbuf, team, tl, active, np, po, maxprim, up.x, X, Y,
+        x_triplet_team<LAB, LC, C::TS, float>(a, txyz, pdesc, rbuf, team, tl, active, np, po, maxprim, up.x, X, Y,
                                               Z, xrow, C::MPAD);
       else
-        x_triplet_team<LAB, LC, C::TS, double>(a, txyz, rdesc, rbuf, team, tl, active, np, po, maxprim, up.x, X,
+        x_triplet_team<LAB, LC, C::TS, double>(a, txyz, pdesc, rbuf, team, tl, active, np, po, maxprim, up.x, X,
                                                Y, Z, xrow, C::MPAD);
     }
     cp_async_commit_wait_all();

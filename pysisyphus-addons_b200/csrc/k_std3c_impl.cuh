@@ -113,11 +113,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_std3c(Std3cArgs a) {
   }
   if constexpr (!C::kPerThread) {
     uchar4* txyz = reinterpret_cast<uchar4*>(Rteam + C::NTRIP * C::kTeamStride);
-    int* rdesc = reinterpret_cast<int*>(txyz + C::NR);
-    for (int i = tid; i < C::NR; i += kThreads) {
-      txyz[i] = *reinterpret_cast<const uchar4*>(a.x.dt.idx->xyz[i]);
-      rdesc[i] = a.x.dt.rdesc[i];
-    }
+    fill_team_tables<C::L>(txyz, reinterpret_cast<int*>(txyz + C::NR), a.x.dt, tid);
   }
   __syncthreads();
   int maxprim = 0, maxu = 0;
@@ -161,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_std3c(Std3cArgs a) {
       }
     } else {
       const uchar4* txyz = reinterpret_cast<const uchar4*>(Rteam + C::NTRIP * C::kTeamStride);
-      const int* rdesc = reinterpret_cast<const int*>(txyz + C::NR);
+      const int* pdesc = reinterpret_cast<const int*>(txyz + C::NR);
       const int team = tid / C::TS, tl = tid - team * C::TS;
       const bool in_team = team < C::NTRIP;
       const int ui = in_team ? team / C::TC : 0, ci = in_team ? team - ui * C::TC : 0;
@@ -175,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_std3c(Std3cArgs a) {
         for (int t = tl; t < C::NH; t += C::TS)
 #pragma unroll
           for (int m = 0; m < C::NC; ++m) xrow[t * C::MPAD + m] = 0.0;
-      x_triplet_team<LAB, LC, C::TS, double>(a.x, txyz, rdesc, rbuf, team, tl, active, active ? c_info[2 * ci] : 0,
+      x_triplet_team<LAB, LC, C::TS, double>(a.x, txyz, pdesc, rbuf, team, tl, active, active ? c_info[2 * ci] : 0,
                                              c_info[2 * ci + 1], maxprim, up.x, up.y - cc.x, up.z - cc.y,
                                              up.w - cc.z, xrow, C::MPAD);
     }
