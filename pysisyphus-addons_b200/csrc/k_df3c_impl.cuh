@@ -417,9 +417,10 @@ __device__ __forceinline__ void x_triplet_team(const Df3cArgs& a, const uchar4* 
       for (int l = 0; l < LC; ++l) pref *= -0.5 / gam;
       // orders n = tl, tl + TS, ...: a team may have fewer lanes than L + 1
       const typename BoysAtT<Real>::type F(a.boys_mode, alpha * RPC2);
+      const double m1 = -2.0 * alpha, m2 = m1 * m1, m4 = m2 * m2, m8 = m4 * m4;
       for (int n = tl; n <= L; n += TS) {
-        double f = pref;
-        for (int k = 0; k < n; ++k) f *= -2.0 * alpha;
+        // pref m1^n, without a chain of n products
+        const double f = (((n & 1) ? pref * m1 : pref) * ((n & 2) ? m2 : 1.0)) * (((n & 4) ? m4 : 1.0) * ((n & 8) ? m8 : 1.0));
         Rn[n] = static_cast<Real>(f) * F(a.dt, n);
       }
     }

@@ -247,9 +247,28 @@ __global__ void __launch_bounds__(32 * kSwWarps) k_schwarz_bra_warp(
   double* Zs = R1 + sw_nr;            // Z_i [NH][nab]
   double* out = Zs + sw_nab * sw_nh;  // A [nab][nab]
   const IndexTables* it = dt.idx;
-  for (int k = lane; k < nab * nab; k += 32) out[k] = 0.0;
   const int u0 = pair_unit0[pair];
   const int nu = sa.y * sb.y;
+  if (nab == 1) {
+    // (ss|ss): one number per unit pair, so the lanes take the unit pairs (45 of
+    // two shells with three primitives each took 50 us one after another)
+    double v = 0.0;
+    for (int idx = lane; idx < nu * (nu + 1) / 2; idx += 32) {
+      int ku = static_cast<int>((sqrtf(8.0f * idx + 1.0f) - 1.0f) * 0.5f);
+      while (ku * (ku + 1) / 2 > idx) --ku;
+      while ((ku + 1) * (ku + 2) / 2 <= idx) ++ku;
+      const int iu = idx - ku * (ku + 1) / 2;
+      const double4 P = U.unit_pP[u0 + iu], Q = U.unit_pP[u0 + ku];
+      const double p = P.x, q = Q.x, pq = p + q, alpha = p * q / pq;
+      const double X = Q.y - P.y, Yd = Q.z - P.z, Z = Q.w - P.w;
+      const double z = kTwoPi52 / (p * q * sqrt(pq)) * boys_n(dt, boys_mode, 0, alpha * (X * X + Yd * Yd + Z * Z));
+      v = fma((ku == iu ? 1.0 : 2.0) * U.esph[U.unit_esph[u0 + iu]], z * U.esph[U.unit_esph[u0 + ku]], v);
+    }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) Qab[pair] = sqrt(sqrt(v * v));  // the norm of the 1 x 1 block, as below
+    return;
+  }
+  for (int k = lane; k < nab * nab; k += 32) out[k] = 0.0;
   for (int iu = 0; iu < nu; ++iu) {
     const double4 P = U.unit_pP[u0 + iu];
     __syncwarp();  // the previous A update has read Z
@@ -713,7 +732,14 @@ constexpr int kBraTChunk = 16;
 __global__ void __launch_bounds__(256) k_bra_prep(DevBasis B, const int2* __restrict__ pair_ab,
                                                   UnitArrays U, BraPrepArgs a) {
   extern __shared__ double smem[];
-  const int slot = a.slot0 + blockIdx.x;
+  if (a.nclass > 0) {  // every class in one launch: this block's class
+    int c = 0;
+    while (c + 1 < a.nclass && static_cast<int>(blockIdx.x) >= a.class_off[c + 1]) ++c;
+    a.slot0 = a.class_off[c];
+    a.n_class = a.class_off[c + 1] - a.slot0;
+    a.g_base = a.class_g[c];
+  }
+  const int slot = a.nclass > 0 ? static_cast<int>(blockIdx.x) : a.slot0 + static_cast<int>(blockIdx.x);
   if (slot >= a.slot_end) return;
   const double q = a.slot_Q[slot];
   if (q * (*a.qmax_aux) < a.thresh) return;  // never reached by any surviving triple
@@ -887,7 +913,7 @@ int launch_bra_prep(const DevBasis& B, const int2* pair_ab, UnitArrays U, const 
   int nab_max = 1;
   for (int la = 0; la <= PA_LMAX; ++la)
     for (int lb = 0; lb <= la; ++lb)
-      if (la + lb == lab) nab_max = max(nab_max, (2 * la + 1) * (2 * lb + 1));
+      if (la + lb == lab || (a.nclass > 0 && la + lb < lab)) nab_max = max(nab_max, (2 * la + 1) * (2 * lb + 1));
   const size_t smem = sizeof(double) * nab_max * (a.nd + kBraTChunk);
   cudaFuncSetAttribute(k_bra_prep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        static_cast<int>(smem));

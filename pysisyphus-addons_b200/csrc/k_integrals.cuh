@@ -26,9 +26,15 @@ struct BraPrepArgs {
   const double* pair_den = nullptr;
   double4* slot_qvl = nullptr;
   double* slot_den = nullptr;
+  // nclass > 0: slots [0, slot_end) of all classes in one launch, class c at
+  // slots [class_off[c], class_off[c + 1]) with its G blocks from class_g[c]
+  int nclass = 0;
+  int class_off[2 * PA_LMAX + 2] = {};
+  long long class_g[2 * PA_LMAX + 1] = {};
 };
 
 size_t schwarz_bra_smem(int lab);
+// lab: the class, or the highest one with nclass > 0.
 int launch_bra_prep(const DevBasis& B, const int2* pair_ab, UnitArrays U, const BraPrepArgs& a,
                     int lab, cudaStream_t s);
 

@@ -552,17 +552,13 @@ __global__ void k_gather_unit_keys(int n, const int* __restrict__ class_unit,
   vals[i] = i;  // input position; class_sort_desc maps it back to the unit
 }
 
-// Sort keys of the auxiliary shells: Q_c, or with QVL screening (qvl != null)
+// Sort key of an auxiliary shell: Q_c, or with QVL screening (qvl != null)
 // the bound max(Q_c, pi sqrt(2) beta_c / (den_min ext_c^(L_c + 1))) of
 // qvl_estimate / Q_ab: beyond the distance ext_ab + ext_c > ext_c the QVL
 // estimate is below Q_ab times the second term, inside it equals Q_ab Q_c. With
 // these keys the staircase of sorted units and shells stays a valid bound.
-__global__ void k_gather_aux_keys(int n, const int* __restrict__ shells, const double* __restrict__ Qc,
-                                  const int4* __restrict__ shell_info, const double2* __restrict__ qvl,
-                                  double den_min, double* keys, int* vals) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int s = shells[i];
+__device__ __forceinline__ double aux_key(int s, const double* __restrict__ Qc, const int4* __restrict__ shell_info,
+                                          const double2* __restrict__ qvl, double den_min) {
   double key = Qc[s];
   if (qvl) {
     const double2 eb = qvl[s];
@@ -570,8 +566,107 @@ __global__ void k_gather_aux_keys(int n, const int* __restrict__ shells, const d
     for (int l = 0; l < shell_info[s].x; ++l) rl *= eb.x;
     key = fmax(key, kPi * sqrt(2.0) * eb.y / (den_min * rl));
   }
-  keys[i] = key;
+  return key;
+}
+__global__ void k_gather_aux_keys(int n, const int* __restrict__ shells, const double* __restrict__ Qc,
+                                  const int4* __restrict__ shell_info, const double2* __restrict__ qvl,
+                                  double den_min, double* keys, int* vals) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  keys[i] = aux_key(shells[i], Qc, shell_info, qvl, den_min);
   vals[i] = i;  // input position; class_sort_desc maps it back to the shell
+}
+
+// Screening lists of small systems in one launch: block 0 sorts the auxiliary
+// shells by key within their class and finds the largest key, block 1 the bra
+// units. The order is class_sort_desc's (class, key descending, input position;
+// keys compared by the bits the radix sort uses), by a bitonic sort in shared
+// memory. The dozen launches it replaces took 0.1 of the 0.19 ms screening of 3
+// to 8 atoms; a block sorts up to kSmallSort entries in 10 to 15 us, and beyond
+// that the radix sorts on all SMs are as fast.
+constexpr int kSmallSort = 4096;
+constexpr int kSmallSortThreads = 1024;
+constexpr size_t kSmallSortSmem = (sizeof(unsigned long long) + sizeof(int)) * kSmallSort;
+struct SmallSortArgs {
+  int n_aux = 0, n_unit = 0, naux_class = 0, nunit_class = 0;
+  const int *aux_shell = nullptr, *aux_off = nullptr, *class_unit = nullptr, *unit_off = nullptr, *unit_pair = nullptr;
+  const double *Qc = nullptr, *Qab = nullptr;
+  const int4* shell_info = nullptr;
+  const double2* qvl = nullptr;
+  double den_min = 1.0;
+  double *aux_Q = nullptr, *slot_Q = nullptr, *qmax = nullptr;
+  int *sorted_aux = nullptr, *sorted_unit = nullptr;
+};
+
+// Bits of a key in descending order, and back.
+__device__ __forceinline__ unsigned long long key_bits(double x) {
+  if (x == 0.0) x = 0.0;  // -0 and 0 tie
+  const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(x));
+  return (u >> 63) ? u : ~u & ~(1ull << 63);
+}
+__device__ __forceinline__ double bits_key(unsigned long long k) {
+  return __longlong_as_double(static_cast<long long>((k >> 63) ? k : ~k & ~(1ull << 63)));
+}
+
+__global__ void __launch_bounds__(kSmallSortThreads) k_small_sort(SmallSortArgs a) {
+  extern __shared__ unsigned long long sk[];        // [kSmallSort]
+  int* sv = reinterpret_cast<int*>(sk + kSmallSort);  // class << 16 | input position
+  __shared__ double s_max[kSmallSortThreads / 32];
+  static_assert(kSmallSort <= 1 << 16, "positions take 16 bits");
+  const bool aux = blockIdx.x == 0;
+  const int n = aux ? a.n_aux : a.n_unit, nseg = aux ? a.naux_class : a.nunit_class;
+  const int* off = aux ? a.aux_off : a.unit_off;
+  if (n <= 0) return;
+  int N = 2;
+  while (N < n) N *= 2;
+  double mx = -1.0;
+  for (int i = threadIdx.x; i < N; i += kSmallSortThreads) {
+    if (i < n) {
+      const double key = aux ? aux_key(a.aux_shell[i], a.Qc, a.shell_info, a.qvl, a.den_min)
+                             : a.Qab[a.unit_pair[a.class_unit[i]]];
+      mx = fmax(mx, key);
+      int c = 0;
+      while (c + 1 < nseg && i >= off[c + 1]) ++c;
+      sk[i] = key_bits(key);
+      sv[i] = c << 16 | i;
+    } else {
+      sk[i] = ~0ull;
+      sv[i] = 0x7fffffff;
+    }
+  }
+  if (aux) {
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  }
+  __syncthreads();
+  if (aux && threadIdx.x == 0) {
+    for (int w = 1; w < kSmallSortThreads / 32; ++w) mx = fmax(mx, s_max[w]);
+    *a.qmax = mx;
+  }
+  for (int k = 2; k <= N; k *= 2)
+    for (int j = k / 2; j > 0; j /= 2) {
+      for (int t = threadIdx.x; t < N / 2; t += kSmallSortThreads) {
+        const int x = 2 * t - (t & (j - 1)), y = x + j;  // x has bit j clear
+        const unsigned long long kx = sk[x], ky = sk[y];
+        const int vx = sv[x], vy = sv[y], cx = vx >> 16, cy = vy >> 16;
+        const bool less = cx != cy ? cx < cy : (kx != ky ? kx < ky : vx < vy);  // x before y
+        if (less != ((x & k) == 0)) {
+          sk[x] = ky;
+          sk[y] = kx;
+          sv[x] = vy;
+          sv[y] = vx;
+        }
+      }
+      __syncthreads();
+    }
+  for (int i = threadIdx.x; i < n; i += kSmallSortThreads) {
+    const int pos = sv[i] & 0xffff;
+    (aux ? a.aux_Q : a.slot_Q)[i] = bits_key(sk[i]);
+    if (aux)
+      a.sorted_aux[i] = a.aux_shell[pos];
+    else
+      a.sorted_unit[i] = a.class_unit[pos];
+  }
 }
 
 // Per auxiliary slot: (Q_c, extent, beta, 0) of the sorted shell (QVL screening).
@@ -802,29 +897,58 @@ int run_screening(const pa_basis_s* orb, const pa_basis_s* aux, const DeviceTabl
                                   o.boys_mode, b.Qab, s);
   *launches += launch_schwarz_aux(aux->dev, dt, o.boys_mode, b.Qc, s);
   const bool qvl = o.screening == PA_SCREEN_QVL;
-  if (nx > 0) {
-    k_gather_aux_keys<<<(nx + 255) / 256, 256, 0, s>>>(nx, aux->d_aux_shell, b.Qc, aux->dev.shell,
-                                                       qvl ? aux->d_aux_qvl : nullptr, orb->qvl_den_min,
-                                                       b.akeys, b.avals);
-    ++*launches;
-    size_t bytes = b.cub_bytes;
-    PA_CUDA(cub::DeviceReduce::Max(b.cub_tmp, bytes, b.akeys, b.qmax, nx, s));  // largest key
-    ++*launches;
-  }
-  if (P.nunits > 0) {
-    k_gather_unit_keys<<<(P.nunits + 255) / 256, 256, 0, s>>>(P.nunits, orb->d_class_unit,
-                                                              orb->d_unit_pair, b.Qab, b.ukeys, b.uvals);
-    ++*launches;
-    *launches += class_sort_desc(b, b.ukeys, b.uvals, orb->d_class_unit, orb->d_class_off, P.lab_max + 1,
-                                 P.nunits, b.slot_Q, b.sorted_unit, s);
-  }
-  if (nx > 0) {
-    *launches += class_sort_desc(b, b.akeys, b.avals, aux->d_aux_shell, aux->d_aux_off, aux->aux.lc_max + 1,
-                                 nx, b.aux_Q, b.sorted_aux, s);
-    if (qvl) {
-      k_aux_slot_qvl<<<(nx + 255) / 256, 256, 0, s>>>(nx, b.sorted_aux, b.Qc, aux->d_aux_qvl, b.aux_slot_qvl);
+  const double2* aux_qvl = qvl ? aux->d_aux_qvl : nullptr;
+  if (nx <= kSmallSort && P.nunits <= kSmallSort) {
+    if (nx > 0 || P.nunits > 0) {
+      SmallSortArgs a;
+      a.n_aux = nx;
+      a.n_unit = P.nunits;
+      a.naux_class = aux->aux.lc_max + 1;
+      a.nunit_class = P.lab_max + 1;
+      a.aux_shell = aux->d_aux_shell;
+      a.aux_off = aux->d_aux_off;
+      a.class_unit = orb->d_class_unit;
+      a.unit_off = orb->d_class_off;
+      a.unit_pair = orb->d_unit_pair;
+      a.Qc = b.Qc;
+      a.Qab = b.Qab;
+      a.shell_info = aux->dev.shell;
+      a.qvl = aux_qvl;
+      a.den_min = orb->qvl_den_min;
+      a.aux_Q = b.aux_Q;
+      a.slot_Q = b.slot_Q;
+      a.qmax = b.qmax;
+      a.sorted_aux = b.sorted_aux;
+      a.sorted_unit = b.sorted_unit;
+      // (the limit without this attribute covers static and dynamic bytes together)
+      PA_CUDA(cudaFuncSetAttribute(k_small_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(kSmallSortSmem)));
+      k_small_sort<<<2, kSmallSortThreads, kSmallSortSmem, s>>>(a);
       ++*launches;
     }
+  } else {
+    if (nx > 0) {
+      k_gather_aux_keys<<<(nx + 255) / 256, 256, 0, s>>>(nx, aux->d_aux_shell, b.Qc, aux->dev.shell, aux_qvl,
+                                                         orb->qvl_den_min, b.akeys, b.avals);
+      ++*launches;
+      size_t bytes = b.cub_bytes;
+      PA_CUDA(cub::DeviceReduce::Max(b.cub_tmp, bytes, b.akeys, b.qmax, nx, s));  // largest key
+      ++*launches;
+    }
+    if (P.nunits > 0) {
+      k_gather_unit_keys<<<(P.nunits + 255) / 256, 256, 0, s>>>(P.nunits, orb->d_class_unit,
+                                                                orb->d_unit_pair, b.Qab, b.ukeys, b.uvals);
+      ++*launches;
+      *launches += class_sort_desc(b, b.ukeys, b.uvals, orb->d_class_unit, orb->d_class_off, P.lab_max + 1,
+                                   P.nunits, b.slot_Q, b.sorted_unit, s);
+    }
+    if (nx > 0)
+      *launches += class_sort_desc(b, b.akeys, b.avals, aux->d_aux_shell, aux->d_aux_off, aux->aux.lc_max + 1,
+                                   nx, b.aux_Q, b.sorted_aux, s);
+  }
+  if (nx > 0 && qvl) {
+    k_aux_slot_qvl<<<(nx + 255) / 256, 256, 0, s>>>(nx, b.sorted_aux, b.Qc, aux->d_aux_qvl, b.aux_slot_qvl);
+    ++*launches;
   }
   return PA_OK;
 }
@@ -850,12 +974,22 @@ void stage_bra_prep(const pa_basis_s* orb, const pa_basis_s* aux, int nd, const 
                     cudaStream_t s, int* launches, cudaEvent_t* ev_lab = nullptr) {
   const PairLists& P = orb->pairs;
   UnitArrays U = unit_arrays(orb, b);
+  // small systems: every class in one launch (a launch costs more than the
+  // shared memory of the largest class takes in occupancy)
+  const bool merged = P.nunits <= kSmallSort;
   for (int lab = 0; lab <= P.lab_max; ++lab) {
     BraPrepArgs a;
-    a.slot0 = P.class_off[lab];
+    if (merged) {
+      if (lab < P.lab_max) continue;
+      a.nclass = P.lab_max + 1;
+      for (int c = 0; c <= a.nclass; ++c) a.class_off[c] = P.class_off[c];
+      for (int c = 0; c < a.nclass; ++c) a.class_g[c] = b.g_off[c];
+    }
+    a.slot0 = merged ? 0 : P.class_off[lab];
     a.slot_end = P.class_off[lab + 1];
     if (a.slot_end <= a.slot0 || nd == 0 || aux->host.shells.empty()) {
-      if (ev_lab) cudaEventRecord(ev_lab[lab], s);
+      if (ev_lab)
+        for (int l = merged ? 0 : lab; l <= lab; ++l) cudaEventRecord(ev_lab[l], s);
       continue;
     }
     a.slot_Q = b.slot_Q;
@@ -879,7 +1013,8 @@ void stage_bra_prep(const pa_basis_s* orb, const pa_basis_s* aux, int nd, const 
       a.slot_den = b.slot_den;
     }
     *launches += launch_bra_prep(orb->dev, orb->d_pair_ab, U, a, lab, s);
-    if (ev_lab) cudaEventRecord(ev_lab[lab], s);
+    if (ev_lab)
+      for (int l = merged ? 0 : lab; l <= lab; ++l) cudaEventRecord(ev_lab[l], s);
   }
 }
 
@@ -1250,6 +1385,7 @@ int df_device(pa_basis orb, pa_basis aux, int ndens, int nbf, const double* d_de
 struct BatchPlan {
   std::vector<long long> sig;
   char* dmem = nullptr;
+  bool owns = true;  // dmem is the plan's own (else the context's arena)
   std::vector<DfBuffers> bufs;
   std::vector<double*> df, gram;
   int* infos = nullptr;      // device: 4 ints per molecule
@@ -1259,7 +1395,7 @@ struct BatchPlan {
   int launches = 0;
   ~BatchPlan() {
     if (exec) cudaGraphExecDestroy(exec);
-    if (dmem) cudaFree(dmem);
+    if (dmem && owns) cudaFree(dmem);
     if (h_infos) cudaFreeHost(h_infos);
   }
 };
@@ -1487,7 +1623,20 @@ int batch_4d(int nmol, const pa_basis* orbs, const pa_basis* auxs, const int* nd
         // room for the class descriptors: at most one per (class, molecule)
         cv.take<Df3cArgs>(class_lab.size() * std::max(nmol, 1));
         cv.take<int>(class_lab.size() * (std::max(nmol, 1) + 1));
-        if (cudaMalloc(&plan->dmem, std::max<size_t>(cv.used, 256)) != cudaSuccess) {
+        // a plan that is not kept for replay lives in the context's arena (the
+        // call is synchronous and holds the context): allocating and freeing
+        // it took 3.6 of 30 ms for 16 molecules
+        plan->owns = use_graph != 0;
+        cudaError_t em = cudaSuccess;
+        if (plan->owns) {
+          em = cudaMalloc(&plan->dmem, std::max<size_t>(cv.used, 256));
+        } else {
+          em = c->arena.reserve(cv.used);
+          plan->dmem = c->arena.base;
+        }
+        if (em != cudaSuccess) {
+          if (plan->owns) plan->dmem = nullptr;
+          plan->owns = false;
           delete plan;
           return fail(PA_ERR_CUDA, "cudaMalloc(batch plan) failed");
         }
