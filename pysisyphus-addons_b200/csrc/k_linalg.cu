@@ -41,15 +41,15 @@ __device__ __forceinline__ void cp_async16_ld(double* smem_dst, const double* gm
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src));
 }
 
-// Cholesky factor of the 64 x 64 block S (lower triangle; row stride NB + 1) in
-// place, its inverse in X (zeros above the diagonal), T scratch; all 256
+// Cholesky factor of the 64 x 64 block S (lower triangle) in
+// place, its inverse in X (undefined right of its 32 x 32 diagonal blocks), T scratch; all 256
 // threads, S complete on entry (after a barrier). Rows and columns from nb on
 // hold the identity. The serial chain is kept short: per pivot one reciprocal
 // square root (the pivot's root follows from it and one Newton correction), per
 // 16-column sub-block
 //  * warp 0 factors the 16 x 16 diagonal sub-block (lane r holds row r, pivots
-//    and L(j, k) move by shuffles; ~345 cycles a pivot, and 490 with two columns
-//    per link through the 2 x 2 determinant: more dependent FP64 operations);
+//    and L(j, k) move by shuffles; two columns per link of the chain, through
+//    the 2 x 2 determinant, was slower: more dependent FP64 operations);
 //  * one thread per row below solves x L11^T = a in registers;
 //  * the trailing lower triangle is updated on the FP64 tensor cores.
 // Inverse: four warps invert the diagonal sub-blocks (lane c holds column c,
@@ -57,32 +57,55 @@ __device__ __forceinline__ void cp_async16_ld(double* smem_dst, const double* gm
 // blocks follow by doubling: X_21 = -X_22 (L_21 X_11) at 16 and at 32 columns,
 // on the FP64 tensor cores as well.
 constexpr int SB = 16;
-__device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X)[NB + 1], double (*T)[NB + 1],
+constexpr int kPanLd = NB + 4;  // 4 (mod 16): conflict-free m8n8k4 fragment loads
+
+// 1 / sqrt(x), x > 0, without a branch: the hardware approximation y and one step
+// of Householder's third-order iteration, y (1 + e / 2 + 3 e^2 / 8) with
+// e = 1 - x y^2 (below 2^-18; the remainder 5 e^3 / 16 is below 2^-55): four
+// dependent operations. Subnormal x is taken times 2^104, infinity gives 0.
+__device__ __forceinline__ double recip_sqrt_step(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double recip_sqrt(double x) {
+  const int hi = __double2hiint(x);
+  const double y = recip_sqrt_step(x), z = recip_sqrt_step(x * 0x1p104) * 0x1p52;
+  return hi < 0x00100000 ? z : (hi >= 0x7ff00000 ? 0.0 : y);
+}
+
+__device__ __forceinline__ void factor_invert_64(double (*S)[kPanLd], double (*X)[kPanLd], double (*T)[kPanLd],
                                                  double* invd, int nb, int pivot0, int* info) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t4 = lane & 3;
-  for (int idx = tid; idx < NB * NB; idx += 256) X[idx >> 6][idx & (NB - 1)] = 0.0;
   for (int k0 = 0; k0 < NB; k0 += SB) {
     if (warp == 0) {
       // lanes 16..31 repeat lanes 0..15 (they only feed the shuffles)
       const int r = lane & (SB - 1);
-      double v[SB];
+      // row r and, apart from it, its diagonal element: the next pivot then
+      // needs no shuffle but its own. No branches: they cost a third of the time
+      double v[SB], dg = S[k0 + r][k0 + r];
+      int bad = -1;  // first non-positive pivot
 #pragma unroll
-      for (int j = 0; j < SB; ++j) v[j] = (j <= r) ? S[k0 + r][k0 + j] : 0.0;
+      for (int j = 0; j < SB; ++j) v[j] = (j < r) ? S[k0 + r][k0 + j] : 0.0;
 #pragma unroll
       for (int k = 0; k < SB; ++k) {
-        double dkk = __shfl_sync(0xffffffffu, v[k], k);
-        if (!(dkk > 0.0)) {
-          if (lane == 0 && k0 + k < nb) atomicCAS(info, 0, pivot0 + k0 + k + 1);
-          dkk = 1.0;  // keep the factor finite; the error is reported through info
-        }
-        const double id = rsqrt(dkk);
-        if (r > k) v[k] *= id;  // L(r, k)
+        double dkk = __shfl_sync(0xffffffffu, dg, k);
+        const bool ok = dkk > 0.0;
+        bad = (!ok && bad < 0) ? k : bad;
+        dkk = ok ? dkk : 1.0;  // keep the factor finite; the error is reported through info
+        const double id = recip_sqrt(dkk);
+        const double l = v[k] * id;  // L(r, k) of the rows below
+        v[k] = r > k ? l : v[k];
+        const double g2 = fma(-l, l, dg);
+        dg = r > k ? g2 : dg;
 #pragma unroll
         for (int j = 1; j < SB; ++j) {  // fixed trip count: j > k folds once k is unrolled
           if (j <= k) continue;
           const double ljk = __shfl_sync(0xffffffffu, v[k], j);  // L(j, k) from lane j
-          if (r >= j) v[j] = fma(-v[k], ljk, v[j]);
+          const double u = fma(-v[k], ljk, v[j]);
+          v[j] = r > j ? u : v[j];
         }
         // sqrt(dkk) from its reciprocal: off the chain of the next pivot
         const double d0 = dkk * id;
@@ -90,6 +113,7 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X
         if (r == k) v[k] = d;
         if (lane == k) invd[k0 + k] = id;
       }
+      if (lane == 0 && bad >= 0 && k0 + bad < nb) atomicCAS(info, 0, pivot0 + k0 + bad + 1);
       if (lane < SB) {
 #pragma unroll
         for (int j = 0; j < SB; ++j)
@@ -117,13 +141,13 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X
     // trailing lower triangle: S -= P P^T of the sub-block's columns P, one 8 x 8
     // tile per warp and turn
     const int m8 = (NB - k0 - SB) / 8, tiles = m8 * (m8 + 1) / 2;  // 8-row tiles, at most 21
+    if (tiles == 0) break;
     int tr[3], tc[3];
     double d[3][2];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       const int t = warp + 8 * q;
-      int bi = 0;
-      while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
+      const int bi = (t >= 1) + (t >= 3) + (t >= 6) + (t >= 10) + (t >= 15);
       tr[q] = k0 + SB + 8 * bi + g;
       tc[q] = k0 + SB + 8 * (t - bi * (bi + 1) / 2);
       d[q][0] = d[q][1] = 0.0;
@@ -155,8 +179,10 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X
     }
     if (lane < SB) {
 #pragma unroll
-      for (int i = 0; i < SB; ++i)
-        if (i >= c) X[o + i][o + c] = x[i];
+      for (int i = 0; i < SB; ++i) {
+        X[o + i][o + c] = i >= c ? x[i] : 0.0;
+        if (warp % 2 == 0) X[o + i][o + SB + c] = 0.0;  // right of it: read as part of the 32-column block
+      }
     }
   }
   __syncthreads();
@@ -203,7 +229,6 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[NB + 1], double (*X
 
 // acc += A^T-layout tile product over [0, kq): As[k][row], Bs[k][col] with row
 // stride kPanLd; warp w owns rows 16 (w % 4) and columns 32 (w / 4).
-constexpr int kPanLd = NB + 4;  // 4 (mod 16): conflict-free m8n8k4 fragment loads
 __device__ __forceinline__ void panel_mma(double (&acc)[2][4][2], const double* As, const double* Bs, int kq) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t4 = lane & 3;
@@ -351,9 +376,9 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
 #pragma unroll
         for (int e = 0; e < 2; ++e) dv[mt][nt][e] -= acc[mt][nt][e];
   }
-  double(*S)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(Bs);
-  double(*X)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(As);
-  double(*T)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(Ds);
+  double(*S)[kPanLd] = reinterpret_cast<double(*)[kPanLd]>(Bs);
+  double(*X)[kPanLd] = reinterpret_cast<double(*)[kPanLd]>(As);
+  double(*T)[kPanLd] = reinterpret_cast<double(*)[kPanLd]>(Ds);
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
@@ -366,8 +391,8 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
   __syncthreads();  // As and Ds are free as well
   factor_invert_64(S, X, T, invd, nr, r0, info);
   double* di = dinv + static_cast<size_t>(i) * NB * NB;
-  for (int idx = tid; idx < NB * NB; idx += 256) {
-    const int r = idx & (NB - 1), j = idx >> 6;
+  for (int q = 0; q < NB * NB / 256; ++q) {  // a warp's 8 x 4 pieces: no bank conflicts, 64 contiguous bytes
+    const int r = 8 * warp + g, j = 4 * q + t4;
     if (r < nr && j <= r) Ai[r + lda * j] = S[r][j];
     di[r + NB * j] = (r < nr && j <= r) ? X[r][j] : 0.0;
   }
