@@ -67,7 +67,7 @@ constexpr int pad_stride(int mp) { return mp + ((20 - mp % 16) % 16); }
 //   0: the largest auxiliary tile (TC shells) that fits two blocks per SM;
 //   1: the tile, at least half as large, that keeps the most lanes busy in the
 //      X build (triplets x lanes per triplet, up to the block's 256 threads);
-//   2: team classes (L > 5) at three blocks per SM: 72 KB of shared memory and
+//   2: team classes at three blocks per SM: 72 KB of shared memory and
 //      80 registers per thread (variant 0 where even one shell does not fit).
 // k_df3c.cu picks the variant per class at run time (default 0).
 template <int LAB, int LC, int V>
@@ -77,7 +77,14 @@ struct Cfg {
   static constexpr int NCC = ncart(LC);
   static constexpr int L = LAB + LC;
   static constexpr int NR = ncum(L);
-  static constexpr bool kPerThread = (L <= 5);
+  // Per-thread X build (R in registers, compile-time indices, every thread of a
+  // triplet redoing R) or by teams (R through shared memory). Per thread wins as
+  // long as R fits or few of its entries are used: up to L = 5 by a factor of 2
+  // against teams ((3,2) 8.4 against 15.3 ms at 200 atoms), at L = 6 for few bra
+  // components ((1,5) 9.2 against 14.9, (2,4) 3.6 against 5.4; but (3,3) 18.2
+  // against 11.7, (4,2) 43.8 against 23.4) and for s auxiliary shells up to L = 7
+  // ((6,0) 2.6 against 4.9, (7,0) 3.8 against 6.6); (2,5) 14.9 against 12.0.
+  static constexpr bool kPerThread = L <= 5 || (L == 6 && LAB <= 2) || (L <= 7 && LC == 0);
   static constexpr int pick_ub(int tc) {
     if (kPerThread) {
       int ub = 64 / NH;
@@ -293,7 +300,7 @@ __device__ __forceinline__ void x_rows_zero(double* xrow0, int mpad, int part) {
     for (int m = 0; m < 2 * LC + 1; ++m) xrow0[th * mpad + m] = 0.0;
 }
 
-// X of one triplet by one thread (L <= 5): Boys, R in registers, solid harmonics.
+// X of one triplet by one thread: Boys, R in registers, solid harmonics.
 template <int LAB, int LC, int NR, int MPAD, int TPT, class Real>
 __device__ __forceinline__ void x_triplet_thread(const Df3cArgs& a, double p, double X, double Y,
                                                  double Z, int np, int po, double* xrow0, int part) {
@@ -323,7 +330,7 @@ __device__ __forceinline__ void x_triplet_thread(const Df3cArgs& a, double p, do
   }
 }
 
-// Recurrence for R by a team (L > 5). The direction rule (x before y before z)
+// Recurrence for R by a team. The direction rule (x before y before z)
 // makes every R_tuv with t > 0 depend on entries of its own (u, v) column alone,
 //   R^n_(t+1)uv = X R^(n+1)_tuv + t R^(n+1)_(t-1)uv,
 // so only the plane t = 0 is built level by level through shared memory (C(L+3, 3)
@@ -391,7 +398,7 @@ __device__ __forceinline__ void hermite_columns(Real X, const Real* plane, const
   }
 }
 
-// X of one triplet by a team of TS threads (L > 5): orders of the Boys
+// X of one triplet by a team of TS threads: orders of the Boys
 // function across lanes, R as above, X rows across the lanes. Every thread of a
 // warp (of a team, for teams larger than a warp) calls this with the same Real
 // (the caller makes the precision choice uniform), so the team barriers pair up.
