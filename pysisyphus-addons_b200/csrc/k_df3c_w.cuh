@@ -196,8 +196,8 @@ __device__ __forceinline__ void x_triplet_thread_w(const Df3cArgs& a, double p, 
   }
 }
 
-// X of one weak triplet by a team of TS threads (L > 5), FP32 throughout; the
-// same level-by-level recurrence as x_triplet_team.
+// X of one weak triplet by a team of TS threads (L > 5), FP32 throughout; R
+// level by level in shared memory.
 template <int LAB, int LC, int TS>
 __device__ __forceinline__ void x_triplet_team_w(const Df3cArgs& a, const uchar4* txyz, const int* rdesc, float* rbuf,
                                                  int team, int tl, bool active, int np, int po, int maxprim, double p,

@@ -258,9 +258,10 @@ __device__ __forceinline__ void panel_mma(double (&acc)[2][4][2], const double* 
 // diagonal block to the next is one launch, and the trailing update of a step
 // runs beside the next step. c = -1: the first diagonal block alone.
 //
-// Bound: latency. Critical path of a step at 40 atoms (n = 2240): ~25 us, block
-// 0's four 64^3 products and the factor; with a launch each for the factor
-// (40 us), the panel and the next column's update a step took ~100 us.
+// Bound: latency of block 0's path, four 64^3 products on one SM (13 of 60
+// thousand cycles) and the factor with its inverse (27 us alone): 36 us a step at
+// n = 448, 45 us at 2240 with the trailing update beside it. With a launch each
+// for the factor (40 us), the panel and the next column's update it was ~100 us.
 constexpr size_t kCholSmem = sizeof(double) * 3 * NB * kPanLd;
 __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, int n, int c, double* dinv,
                                                       int* info) {

@@ -388,6 +388,11 @@ struct pa_basis_s {
   int* d_class_off = nullptr;    // [lab_max + 2]
   int* d_class_pair = nullptr;   // pairs grouped by Lab
   int* d_pair_class_off = nullptr;  // [lab_max + 2]
+  // one-center pairs (a, a) alone, for the std tensors that need no others
+  // (classes, units and pairs of `diag`; ids and offsets are those of `pairs`)
+  pa::PairLists diag;
+  int* d_diag_unit = nullptr;
+  int* d_diag_pair = nullptr;
   int* d_aux_shell = nullptr;    // aux shells grouped by L
   int* d_aux_off = nullptr;      // [lc_max + 2]
   // QVL screener data: per shell (as an auxiliary basis) and per shell pair
@@ -1232,8 +1237,25 @@ int ensure_pairs(pa_basis b) {
   std::lock_guard<std::mutex> lk(b->pair_mu);
   if (b->pairs_ready) return PA_OK;
   if (b->host.lmax > PA_LMAX) return fail(PA_ERR_LMAX, "orbital basis L above the compiled maximum");
-  PairLists P;
+  PairLists P, D;
   build_pair_lists(b->host, &P);
+  D.lab_max = P.lab_max;
+  D.class_off.assign(P.lab_max + 2, 0);
+  D.pair_class_off.assign(P.lab_max + 2, 0);
+  const int nsh = static_cast<int>(b->host.shells.size());
+  for (int lab = 0; lab <= P.lab_max; ++lab) {
+    for (int a = 0; a < nsh; ++a) {
+      const HostShell& sa = b->host.shells[a];
+      if (2 * sa.L != lab) continue;
+      const int pair = a * (a + 1) / 2 + a;
+      D.class_pair.push_back(pair);
+      for (int u = 0; u < sa.nprim * sa.nprim; ++u) D.class_unit.push_back(P.pair_unit0[pair] + u);
+    }
+    D.pair_class_off[lab + 1] = static_cast<int>(D.class_pair.size());
+    D.class_off[lab + 1] = static_cast<int>(D.class_unit.size());
+  }
+  D.npairs = static_cast<int>(D.class_pair.size());
+  D.nunits = static_cast<int>(D.class_unit.size());
   Carver cnt;
   char* dpair = nullptr;
   for (int pass = 0; pass < 2; ++pass) {
@@ -1252,6 +1274,8 @@ int ensure_pairs(pa_basis b) {
     b->d_class_off = cnt.take<int>(P.class_off.size());
     b->d_class_pair = cnt.take<int>(P.class_pair.size());
     b->d_pair_class_off = cnt.take<int>(P.pair_class_off.size());
+    b->d_diag_unit = cnt.take<int>(D.class_unit.size());
+    b->d_diag_pair = cnt.take<int>(D.class_pair.size());
   }
   std::vector<char> stage(cnt.used);
   auto put = [&](const void* dst, const void* src, size_t bytes) {
@@ -1266,12 +1290,15 @@ int ensure_pairs(pa_basis b) {
   put(b->d_class_off, P.class_off.data(), sizeof(int) * P.class_off.size());
   put(b->d_class_pair, P.class_pair.data(), sizeof(int) * P.class_pair.size());
   put(b->d_pair_class_off, P.pair_class_off.data(), sizeof(int) * P.pair_class_off.size());
+  put(b->d_diag_unit, D.class_unit.data(), sizeof(int) * D.class_unit.size());
+  put(b->d_diag_pair, D.class_pair.data(), sizeof(int) * D.class_pair.size());
   const cudaError_t e = cudaMemcpy(dpair, stage.data(), cnt.used, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(dpair);
     return fail(PA_ERR_CUDA, std::string("pair-list upload: ") + cudaGetErrorString(e));
   }
   b->pairs = std::move(P);
+  b->diag = std::move(D);
   b->dpair = dpair;
   b->pairs_ready = true;
   return PA_OK;
@@ -1963,15 +1990,20 @@ int std_device(pa_basis orb, pa_basis aux, int kind, int nmos, const double* d_m
   launches += add_diagonal(b.M, naux, o.metric_shift, s2);
   launches += cholesky_lower(b.M, naux, b.info, b.lawork, s2, &c->la2);
   PA_CUDA(cudaEventRecord(c->m1, s2));
-  // Schwarz vectors (screener%init, common/screening.f90:101-163)
+  // Schwarz vectors (screener%init, common/screening.f90:101-163); df1c and
+  // eri2c use the one-center pairs only (60 atoms: 72 000 pairs become 380, and
+  // the screening 2.3 ms becomes launches)
   UnitArrays U;
   U.unit_pair = orb->d_unit_pair;
   U.unit_prims = orb->d_unit_prims;
   U.unit_esph = orb->d_unit_esph;
   U.unit_pP = b.pP;
   U.esph = b.esph;
-  launches += launch_unit_setup(orb->dev, orb->d_pair_ab, orb->d_class_unit, P, U, dt, s);
-  launches += launch_schwarz_bra(orb->dev, orb->d_pair_ab, orb->d_pair_unit0, orb->d_class_pair, P, U, dt,
+  const bool one_center = kind != kStdDf2cMo;
+  launches += launch_unit_setup(orb->dev, orb->d_pair_ab, one_center ? orb->d_diag_unit : orb->d_class_unit,
+                                one_center ? orb->diag : P, U, dt, s);
+  launches += launch_schwarz_bra(orb->dev, orb->d_pair_ab, orb->d_pair_unit0,
+                                 one_center ? orb->d_diag_pair : orb->d_class_pair, one_center ? orb->diag : P, U, dt,
                                  o.boys_mode, b.Qab, s);
   launches += launch_schwarz_aux(aux->dev, dt, o.boys_mode, b.Qc, s);
   PA_CUDA(cudaEventRecord(c->ph[0], s));
