@@ -415,7 +415,10 @@ __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, 
 // Bound: for few columns the solving blocks' chain of loads and barriers, so
 // R = 2 with every fragment of a step in registers (one block per SM); for many
 // the FP64 tensor pipe, so R = 4 (half the passes over B, two blocks per SM).
-constexpr int kTrsmFew = 192;  // densities of up to 19 states
+// Measured (n = 2240 / 3360, R = 2 against 4): 64 columns 213 against 223 / 321
+// against 338 us, 128: 214, 227 / 382, 385, 192: 248, 235 / 456, 426, 1000: 699,
+// 391 / 1534, 802.
+constexpr int kTrsmFew = 128;
 constexpr int kTrsmLdx = 12;  // 4 or 12 (mod 16): conflict-free fragment loads
 constexpr size_t trsm_smem(int nt, int nblk) {
   return sizeof(double) * std::max(nblk * NB * (8 * nt + 4), nblk * NB * kTrsmLdx + 2 * NB * kTrsmLdx);

@@ -587,8 +587,9 @@ __global__ void k_gather_aux_keys(int n, const int* __restrict__ shells, const d
 // units. The order is class_sort_desc's (class, key descending, input position;
 // keys compared by the bits the radix sort uses), by a bitonic sort in shared
 // memory. The dozen launches it replaces took 0.1 of the 0.19 ms screening of 3
-// to 8 atoms; a block sorts up to kSmallSort entries in 10 to 15 us, and beyond
-// that the radix sorts on all SMs are as fast.
+// to 8 atoms; the sort itself takes 30 us at 8 atoms (1800 primitive pairs), the
+// radix-sort kernels took 58 us without their launches. The limit is what 48 KB of
+// shared memory hold; larger lists go to the radix sorts on all SMs.
 constexpr int kSmallSort = 4096;
 constexpr int kSmallSortThreads = 1024;
 constexpr size_t kSmallSortSmem = (sizeof(unsigned long long) + sizeof(int)) * kSmallSort;

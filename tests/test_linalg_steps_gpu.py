@@ -38,7 +38,7 @@ def test_factor_and_solve_block_edges(n):
 
 
 @pytest.mark.parametrize("n", [130, 400])
-@pytest.mark.parametrize("nrhs", [1, 7, 8, 9, 40, 41, 64, 192, 193, 300])
+@pytest.mark.parametrize("nrhs", [1, 7, 8, 9, 40, 41, 64, 128, 129, 192, 193, 300])
 def test_solve_column_counts(n, nrhs):
     A = spd(n, 7)
     B = np.random.default_rng(nrhs).normal(size=(n, nrhs))
