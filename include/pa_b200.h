@@ -298,6 +298,12 @@ int pa_cholesky_solve(int n, double* A, int nrhs, double* B);
  * BF16 slices per operand, six slice products accumulated in FP32 in tensor
  * memory). 1 <= m <= 128, 1 <= n <= 48, 1 <= k <= 128. Synchronous. */
 int pa_split_product_check(int m, int n, int k, const double* A, const double* B, double* C);
+/* Order of the launches of the Cholesky factorization of an n x n matrix
+ * (1 <= n <= 16384) on its two streams, from a graph that is captured and not
+ * launched: *missing = orders that a step or a trailing update needs and does not
+ * have (0), *pairs = trailing updates that another step follows, *apart = those of
+ * them that may run beside that step (all). */
+int pa_cholesky_order_check(int n, int* missing, int* apart, int* pairs);
 
 /* The estimator study (replaces intor/benchmark_wrapper.f90:13-37,
  * f_benchmark_int3c2e, same arguments): prints the basis sizes, the time and

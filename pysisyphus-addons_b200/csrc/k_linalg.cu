@@ -259,9 +259,10 @@ __device__ __forceinline__ void panel_mma(double (&acc)[2][4][2], const double* 
 // runs beside the next step. c = -1: the first diagonal block alone.
 //
 // Bound: latency of block 0's path, four 64^3 products on one SM (13 of 60
-// thousand cycles) and the factor with its inverse (27 us alone): 36 us a step at
-// n = 448, 45 us at 2240 with the trailing update beside it. With a launch each
-// for the factor (40 us), the panel and the next column's update it was ~100 us.
+// thousand cycles) and the factor with its inverse (27 us alone). With the trailing
+// update beside the next step 33 us a step at n = 448, 37 us at 2240 and 39 us at
+// 3360; in one stream, step, update, step, 37, 45 and 51 us. With a launch each for
+// the factor (40 us), the panel and the next column's update it was ~100 us.
 constexpr size_t kCholSmem = sizeof(double) * 3 * NB * kPanLd;
 __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, int n, int c, double* dinv,
                                                       int* info) {
@@ -859,12 +860,13 @@ int cholesky_lower(double* A, int n, int* d_info, double* work, cudaStream_t s,
   cudaMemsetAsync(d_info, 0, sizeof(int), s);
   const int nblk = (n + NB - 1) / NB;
   // Step c (k_chol_step) on s; its trailing update of block columns c + 2.. on
-  // the aux stream beside step c + 1, which needs the update of step c - 1 only.
+  // the aux stream beside step c + 1, which takes column c itself and needs the
+  // updates up to that of step c - 1 only.
   bool pending[2] = {false, false};  // an update of a step of this parity is queued on la->aux
   for (int c = -1; c + 1 < nblk; ++c) {
-    if (la && c >= 1 && pending[(c + 1) & 1]) {
-      cudaStreamWaitEvent(s, la->ev_rest[(c + 1) & 1], 0);  // update of step c - 1
-      pending[(c + 1) & 1] = false;
+    if (la && c >= 2 && pending[c & 1]) {
+      cudaStreamWaitEvent(s, la->ev_rest[c & 1], 0);  // update of step c - 2
+      pending[c & 1] = false;
     }
     k_chol_step<<<c < 0 ? 1 : nblk - 1 - c, 256, kCholSmem, s>>>(A, n, n, c, work, d_info);
     ++launches;

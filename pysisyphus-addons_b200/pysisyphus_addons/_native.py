@@ -138,6 +138,7 @@ SIGNATURES = {
     "pa_eval_densities": _BASIS + [_i, _pd, _i, _i, _pd, _i, _pd, _i, _d],
     "pa_eval_prim_density": [_i, _i, _i, _pi, _pd, _pd, _pd, _i, _d, _pd],
     "pa_split_product_check": [_i, _i, _i, _pd, _pd, _pd],
+    "pa_cholesky_order_check": [_i, _pi, _pi, _pi],
 }
 
 _lib = None
