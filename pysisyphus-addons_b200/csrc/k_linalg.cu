@@ -45,8 +45,8 @@ __device__ __forceinline__ void cp_async16_ld(double* smem_dst, const double* gm
 // place, its inverse in X (undefined right of its 32 x 32 diagonal blocks), T scratch; all 256
 // threads, S complete on entry (after a barrier). Rows and columns from nb on
 // hold the identity. The serial chain is kept short: per pivot one reciprocal
-// square root (the pivot's root follows from it and one Newton correction), per
-// 16-column sub-block
+// square root (CUDA's; the roots follow after it, one per lane), per 16-column
+// sub-block
 //  * warp 0 factors the 16 x 16 diagonal sub-block (lane r holds row r, pivots
 //    and L(j, k) move by shuffles; two columns per link of the chain, through
 //    the 2 x 2 determinant, was slower: more dependent FP64 operations);
@@ -59,22 +59,6 @@ __device__ __forceinline__ void cp_async16_ld(double* smem_dst, const double* gm
 constexpr int SB = 16;
 constexpr int kPanLd = NB + 4;  // 4 (mod 16): conflict-free m8n8k4 fragment loads
 
-// 1 / sqrt(x), x > 0, without a branch: the hardware approximation y and one step
-// of Householder's third-order iteration, y (1 + e / 2 + 3 e^2 / 8) with
-// e = 1 - x y^2 (below 2^-18; the remainder 5 e^3 / 16 is below 2^-55): four
-// dependent operations. Subnormal x is taken times 2^104, infinity gives 0.
-__device__ __forceinline__ double recip_sqrt_step(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-__device__ __forceinline__ double recip_sqrt(double x) {
-  const int hi = __double2hiint(x);
-  const double y = recip_sqrt_step(x), z = recip_sqrt_step(x * 0x1p104) * 0x1p52;
-  return hi < 0x00100000 ? z : (hi >= 0x7ff00000 ? 0.0 : y);
-}
-
 __device__ __forceinline__ void factor_invert_64(double (*S)[kPanLd], double (*X)[kPanLd], double (*T)[kPanLd],
                                                  double* invd, int nb, int pivot0, int* info) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -84,7 +68,7 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[kPanLd], double (*X
       // lanes 16..31 repeat lanes 0..15 (they only feed the shuffles)
       const int r = lane & (SB - 1);
       // row r and, apart from it, its diagonal element: the next pivot then
-      // needs no shuffle but its own. No branches: they cost a third of the time
+      // needs no shuffle but its own. No branches on r: they cost a third of the time
       double v[SB], dg = S[k0 + r][k0 + r];
       int bad = -1;  // first non-positive pivot
 #pragma unroll
@@ -95,7 +79,7 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[kPanLd], double (*X
         const bool ok = dkk > 0.0;
         bad = (!ok && bad < 0) ? k : bad;
         dkk = ok ? dkk : 1.0;  // keep the factor finite; the error is reported through info
-        const double id = recip_sqrt(dkk);
+        const double id = rsqrt(dkk);
         const double l = v[k] * id;  // L(r, k) of the rows below
         v[k] = r > k ? l : v[k];
         const double g2 = fma(-l, l, dg);
@@ -107,17 +91,14 @@ __device__ __forceinline__ void factor_invert_64(double (*S)[kPanLd], double (*X
           const double u = fma(-v[k], ljk, v[j]);
           v[j] = r > j ? u : v[j];
         }
-        // sqrt(dkk) from its reciprocal: off the chain of the next pivot
-        const double d0 = dkk * id;
-        const double d = isinf(dkk) ? dkk : fma(fma(-d0, d0, dkk), 0.5 * id, d0);
-        if (r == k) v[k] = d;
         if (lane == k) invd[k0 + k] = id;
       }
       if (lane == 0 && bad >= 0 && k0 + bad < nb) atomicCAS(info, 0, pivot0 + k0 + bad + 1);
       if (lane < SB) {
 #pragma unroll
         for (int j = 0; j < SB; ++j)
-          if (j <= r) S[k0 + r][k0 + j] = v[j];
+          if (j < r) S[k0 + r][k0 + j] = v[j];
+        S[k0 + r][k0 + r] = sqrt(dg > 0.0 ? dg : 1.0);  // dg has stayed this row's pivot
       }
     }
     __syncthreads();
@@ -258,11 +239,12 @@ __device__ __forceinline__ void panel_mma(double (&acc)[2][4][2], const double* 
 // diagonal block to the next is one launch, and the trailing update of a step
 // runs beside the next step. c = -1: the first diagonal block alone.
 //
-// Bound: latency of block 0's path, four 64^3 products on one SM (13 of 60
-// thousand cycles) and the factor with its inverse (27 us alone). With the trailing
-// update beside the next step 33 us a step at n = 448, 37 us at 2240 and 39 us at
-// 3360; in one stream, step, update, step, 37, 45 and 51 us. With a launch each for
-// the factor (40 us), the panel and the next column's update it was ~100 us.
+// Bound: latency of block 0's path, four 64^3 products on one SM (13 thousand
+// cycles) and the factor with its inverse (25 us alone; 27 with a reciprocal root
+// written out here and the roots on the chain). With the trailing update beside the
+// next step 30 us a step at n = 448, 33 us at 2240 and 36 us at 3360; in one
+// stream, step, update, step, 33, 41 and 47 us. With a launch each for the factor
+// (40 us), the panel and the next column's update it was ~100 us.
 constexpr size_t kCholSmem = sizeof(double) * 3 * NB * kPanLd;
 __global__ void __launch_bounds__(256, 2) k_chol_step(double* A, long long lda, int n, int c, double* dinv,
                                                       int* info) {
