@@ -158,7 +158,10 @@ int pa_get_mixed_kernels(void);
 int pa_set_class_grid(int mode);
 /* The f_* entry points keep the device copies (with the shell-pair lists) of
  * the last 8 bases they were given, for later calls with byte-identical basis
- * arrays on the same device; pa_basis_cache_clear frees them. pa_get_device
+ * arrays on the same device. Calls also leave their scratch memory mapped for the
+ * next one, per device as much as the largest call took (a batch without a graph
+ * at most 4 GiB and a quarter; grid densities 512 MiB).
+ * pa_basis_cache_clear gives back both, on every device. pa_get_device
  * gives the CUDA device of the calling thread, on which calls run. */
 int pa_basis_cache_clear(void);
 int pa_get_device(int* device);

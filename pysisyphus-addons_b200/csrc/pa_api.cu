@@ -343,15 +343,20 @@ void build_qvl_aux(const HostBasis& b, std::vector<double2>* ext_beta) {
   }
 }
 
+cudaError_t Arena::release() {
+  if (!base) return cudaSuccess;
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) return e;
+  cudaFree(base);
+  base = nullptr;
+  cap = 0;
+  return cudaSuccess;
+}
+
 cudaError_t Arena::reserve(size_t bytes) {
   if (bytes <= cap) return cudaSuccess;
-  if (base) {
-    cudaError_t e = cudaDeviceSynchronize();
-    if (e != cudaSuccess) return e;
-    cudaFree(base);
-    base = nullptr;
-    cap = 0;
-  }
+  const cudaError_t er = release();
+  if (er != cudaSuccess) return er;
   const size_t want = bytes + bytes / 4 + (64 << 20);
   cudaError_t e = cudaMalloc(&base, want);
   if (e != cudaSuccess) {
@@ -1427,6 +1432,7 @@ struct BatchPlan {
     if (h_infos) cudaFreeHost(h_infos);
   }
 };
+constexpr size_t kBatchKeep = size_t(4) << 30;  // arena bytes a batch without a graph may leave behind
 
 struct BatchMol {
   pa_basis orb, aux;
@@ -1653,15 +1659,20 @@ int batch_4d(int nmol, const pa_basis* orbs, const pa_basis* auxs, const int* nd
         cv.take<int>(class_lab.size() * (std::max(nmol, 1) + 1));
         // a plan that is not kept for replay lives in the context's arena (the
         // call is synchronous and holds the context): allocating and freeing
-        // it took 3.6 of 30 ms for 16 molecules
-        plan->owns = use_graph != 0;
-        cudaError_t em = cudaSuccess;
-        if (plan->owns) {
-          em = cudaMalloc(&plan->dmem, std::max<size_t>(cv.used, 256));
-        } else {
+        // it took 3.6 of 30 ms for 16 molecules (2.5 GB). A larger plan than
+        // kBatchKeep is only put there when it fits as it is, so that a batch
+        // leaves no more than that behind
+        plan->owns = use_graph != 0 || (cv.used > kBatchKeep && cv.used > c->arena.cap);
+        cudaError_t em = cudaErrorMemoryAllocation;
+        if (!plan->owns) {
           em = c->arena.reserve(cv.used);
           plan->dmem = c->arena.base;
+          if (em != cudaSuccess) {  // the arena grows by more than it needs
+            cudaGetLastError();
+            plan->owns = true;
+          }
         }
+        if (plan->owns) em = cudaMalloc(&plan->dmem, std::max<size_t>(cv.used, 256));
         if (em != cudaSuccess) {
           if (plan->owns) plan->dmem = nullptr;
           plan->owns = false;
@@ -2315,6 +2326,17 @@ int pa_basis_cache_clear(void) {
     cache.entries.clear();
   }
   release_grid_pools();
+  std::vector<Ctx*> ctx;
+  {
+    std::lock_guard<std::mutex> lk(g_ctx_mu);
+    ctx = g_ctx;
+  }
+  for (Ctx* c : ctx) {
+    if (!c) continue;
+    std::lock_guard<std::mutex> lk(c->mu);  // calls are synchronous: nothing of theirs is in flight
+    PA_CUDA(c->arena.release());
+    PA_CUDA(cudaMemPoolTrimTo(c->pool, 0));
+  }
   return PA_OK;
 }
 

@@ -117,6 +117,7 @@ struct Arena {
   char* base = nullptr;
   size_t cap = 0, used = 0;
   cudaError_t reserve(size_t bytes);
+  cudaError_t release();
   void reset() { used = 0; }
   template <class T>
   T* take(size_t count) {

@@ -367,7 +367,8 @@ def cached_basis(shells, role="orbital"):
 
 
 def clear_basis_cache():
-    """Frees the cached device bases of this module and of the f_* entry points."""
+    """Frees the cached device bases of this module and of the f_* entry points,
+    and the scratch memory the library keeps between calls."""
     with _basis_lock:
         _basis_cache.clear()
     check(load().pa_basis_cache_clear())
