@@ -344,7 +344,12 @@ int pa_eval_densities(int nshells, int ndata, const int* bas_centers, const int*
  * ls_inds(2, nprims) = (L, 0-based Cartesian start), primdata(5, nprims) =
  * (coefficient, exponent, x, y, z), coords3d(3, npoints), P(nbfs, nbfs),
  * rho(npoints) written. L up to 4 (the reference's g prefactors fill 14 of
- * the 15 components; these are all 15). Host buffers; synchronous. */
+ * the 15 components; these are all 15). The reference leaves a pair out at points
+ * with p |r - P|^2 >= 36 (:13). Finite input with positive exponents takes a
+ * product form that sums those terms (up to 1e-10 of the pair's largest value) and
+ * drops primitives beyond an exponent of 80; other input, if only in one element
+ * of P, takes a kernel that leaves them out as the reference does. Host buffers;
+ * synchronous. */
 int f_eval_prim_density(int nprims, int npoints, int nbfs, const int* ls_inds, const double* primdata,
                         const double* coords3d, const double* P, double sw, double* rho);
 /* The same with P in `layout`. */
