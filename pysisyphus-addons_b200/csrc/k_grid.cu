@@ -733,12 +733,10 @@ int eval_densities(int nshells, int ndata, const int* bas_centers, const int* ba
 
 template <int NT>
 int launch_prim_product(PrimArgs a, Staged& tab, size_t o_prim, size_t o_fn, const double* coords3d, const double* P,
-                        size_t nP, double* rho, CallBuf& buf) {
+                        size_t nP, double* rho, int sms, CallBuf& buf) {
   constexpr int pts = QuadTile<NT>::P;
   a.blk = pts;
   a.nblks = (a.npoints + pts - 1) / pts;
-  int sms = 148;
-  PA_GRID_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, buf.dev));
   const size_t slot_bytes = sizeof(double) * static_cast<size_t>(a.nfn) * pts + sizeof(int) * (a.nfn + a.nprim);
   int slots = std::min(a.nblks, 2 * sms);
   slots = std::max(1, std::min<int>(slots, static_cast<int>((size_t(1) << 30) / std::max<size_t>(slot_bytes, 1))));
@@ -830,9 +828,11 @@ int eval_prim_density(int nprims, int npoints, int nbfs, const int* ls_inds, con
     a.si = si;
     a.sj = sj;
     a.sw = sw;
+    int sms = 148;
+    PA_GRID_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, buf.dev));
     // 64 points per block, 32 where 64 would leave SMs without a block
-    if (npoints < 64 * 148) return launch_prim_product<2>(a, tab, o_prim, o_fn, coords3d, P, nP, rho, buf);
-    return launch_prim_product<4>(a, tab, o_prim, o_fn, coords3d, P, nP, rho, buf);
+    if (npoints < 64 * sms) return launch_prim_product<2>(a, tab, o_prim, o_fn, coords3d, P, nP, rho, sms, buf);
+    return launch_prim_product<4>(a, tab, o_prim, o_fn, coords3d, P, nP, rho, sms, buf);
   }
   std::vector<PrimPairG> pairs;
   for (int ai = 0; ai < nprims; ++ai) {
