@@ -8,8 +8,8 @@
 //    followed by dtrmm("L","L","N","N"), diabatization/intor.f90:198: the
 //    explicit inverse is never formed);
 //  * a tiled FP64 GEMM C := beta C + alpha op(A) op(B) on the FP64 tensor
-//    cores with optional lower triangular A, used by all of the above and by
-//    the Coulomb-tensor Gram matrix;
+//    cores, used by the sTDDFT tensors and by the Gram matrix of the Coulomb
+//    tensor for many densities;
 //  * the 8-fold-symmetric scatter of the Coulomb tensor
 //    (diabatization/intor.f90:241-269).
 #include <algorithm>
@@ -565,15 +565,13 @@ __global__ void __launch_bounds__(256, R == 2 ? 1 : 2) k_trsm_step(const double*
 // tensor cores (mma.sync m8n8k4): warp w owns rows 16 (w % 4) .. + 16 and
 // columns 32 (w / 4) .. + 32 of the tile.
 // lower_c: skip output tiles strictly above the diagonal (and entries above it).
-// lower_a: A (not transposed) is lower triangular; entries above its diagonal
-//          are treated as zero whatever the storage holds.
 constexpr int TM = 64, TN = 64, TK = 16;
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(256) k_gemm(int m, int n, int k, double alpha,
                                               const double* __restrict__ A, long long lda,
                                               const double* __restrict__ B, long long ldb,
                                               double beta, double* C, long long ldc,
-                                              int lower_c, int lower_a) {
+                                              int lower_c) {
   const int bi = blockIdx.x, bj = blockIdx.y;
   if (lower_c && bj > bi) return;
   __shared__ double As[TK][TM + 1];
@@ -583,9 +581,7 @@ __global__ void __launch_bounds__(256) k_gemm(int m, int n, int k, double alpha,
   const int wm = (warp & 3) * 16, wn = (warp >> 2) * 32;
   const int i0 = bi * TM, j0 = bj * TN;
   double acc[2][4][2] = {};
-  // with a lower triangular A, columns k > i0 + TM - 1 contribute nothing
-  const int kend = (lower_a && !TA) ? min(k, i0 + TM) : k;
-  for (int kk = 0; kk < kend; kk += TK) {
+  for (int kk = 0; kk < k; kk += TK) {
     for (int idx = threadIdx.x; idx < TK * TM; idx += 256) {
       int r, c;  // r in tile rows (m), c in k
       if (TA) {  // A stored k x m: op(A)(r, c) = A[c + lda * r]
@@ -597,7 +593,7 @@ __global__ void __launch_bounds__(256) k_gemm(int m, int n, int k, double alpha,
       }
       const int gi = i0 + r, gk = kk + c;
       double v = 0.0;
-      if (gi < m && gk < k && (!lower_a || TA || gi >= gk)) v = TA ? A[gk + lda * gi] : A[gi + lda * gk];
+      if (gi < m && gk < k) v = TA ? A[gk + lda * gi] : A[gi + lda * gk];
       As[c][r] = v;
     }
     for (int idx = threadIdx.x; idx < TK * TN; idx += 256) {
@@ -791,23 +787,6 @@ __global__ void k_add_diagonal(double* A, int n, double shift) {
   if (i < n) A[i + static_cast<long long>(n) * i] += shift;
 }
 
-int gemm_impl(bool ta, bool tb, int m, int n, int k, double alpha, const double* A, long long lda,
-              const double* B, long long ldb, double beta, double* C, long long ldc, bool lower_c,
-              bool lower_a, cudaStream_t s) {
-  if (m <= 0 || n <= 0) return 0;
-  dim3 grid((m + TM - 1) / TM, (n + TN - 1) / TN);
-  const int lc = lower_c ? 1 : 0, la = lower_a ? 1 : 0;
-  if (!ta && !tb)
-    k_gemm<false, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc, la);
-  else if (!ta && tb)
-    k_gemm<false, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc, la);
-  else if (ta && !tb)
-    k_gemm<true, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc, la);
-  else
-    k_gemm<true, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc, la);
-  return 1;
-}
-
 // C -= P P^T on the lower part of C (m x m) without its first diagonal tile, P m x k (k <= NB).
 int syrk_update(int m, int k, const double* P, long long ldp, double* C, long long ldc, cudaStream_t s) {
   if (m <= 0) return 0;
@@ -825,7 +804,18 @@ int syrk_update(int m, int k, const double* P, long long ldp, double* C, long lo
 int gemm(bool ta, bool tb, int m, int n, int k, double alpha, const double* A, long long lda,
          const double* B, long long ldb, double beta, double* C, long long ldc, bool lower_only,
          cudaStream_t s) {
-  return gemm_impl(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only, false, s);
+  if (m <= 0 || n <= 0) return 0;
+  dim3 grid((m + TM - 1) / TM, (n + TN - 1) / TN);
+  const int lc = lower_only ? 1 : 0;
+  if (!ta && !tb)
+    k_gemm<false, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc);
+  else if (!ta && tb)
+    k_gemm<false, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc);
+  else if (ta && !tb)
+    k_gemm<true, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc);
+  else
+    k_gemm<true, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lc);
+  return 1;
 }
 
 size_t linalg_workspace_doubles(int n) {
