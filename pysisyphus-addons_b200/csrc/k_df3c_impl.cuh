@@ -25,8 +25,8 @@
 //      memory while
 //   2. X of the UB x TC triplets is built into shared memory: the Boys function,
 //      the Hermite recurrence for R and the solid-harmonic contraction --
-//      per thread with R in registers and compile-time indices for L <= 5, by
-//      thread teams with R in shared memory above;
+//      per thread with R in registers and compile-time indices for small L
+//      (Cfg::kPerThread), by thread teams with R in shared memory above;
 //   3. the update acc[aux fn][d] += X^T G runs on the FP64 tensor cores
 //      (mma.sync m8n8k4 f64), accumulators in registers.
 // Each block writes its partial sums to a per-chunk slab; k_df3c_reduce sums the

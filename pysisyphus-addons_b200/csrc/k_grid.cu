@@ -37,10 +37,12 @@
 // Non-finite densities, coefficients or centers and exponents that are not
 // positive take k_prim_density, which evaluates the reference's pairs one by one.
 //
-// Bound: the FP64 tensor pipe over the surviving tiles, the exponentials for
-// few functions. Measured on B200: 64^3 points around 40 atoms 0.97 ms, 2.0 ms with
-// a broadcast shared-memory load per multiply-add; primitive density of 20 atoms
-// at 60 007 points 0.58 ms, 5.2 ms pair by pair.
+// Bound: latency, of the loads and tests that make up the weight tiles and of the
+// exponentials, at 16 warps per SM (counters: FP64 tensor pipe 13 % busy in the grid
+// density and 27 % in the primitive density, FP64 pipe 9 and 10 %). Measured on
+// B200: 64^3 points around 40 atoms 0.97 ms, 2.0 ms with a broadcast shared-memory
+// load per multiply-add; primitive density of 20 atoms at 60 007 points 0.58 ms,
+// 5.2 ms pair by pair.
 #include <cuda_runtime.h>
 
 #include <algorithm>
