@@ -2331,12 +2331,19 @@ int pa_basis_cache_clear(void) {
     std::lock_guard<std::mutex> lk(g_ctx_mu);
     ctx = g_ctx;
   }
-  for (Ctx* c : ctx) {
+  int cur = 0;
+  cudaError_t e = cudaSuccess;
+  for (size_t dev = 0; dev < ctx.size(); ++dev) {
+    Ctx* c = ctx[dev];
     if (!c) continue;
-    std::lock_guard<std::mutex> lk(c->mu);  // calls are synchronous: nothing of theirs is in flight
-    PA_CUDA(c->arena.release());
-    PA_CUDA(cudaMemPoolTrimTo(c->pool, 0));
+    std::lock_guard<std::mutex> lk(c->mu);
+    if (e == cudaSuccess) e = cudaGetDevice(&cur);
+    if (e == cudaSuccess) e = cudaSetDevice(static_cast<int>(dev));  // the arena waits for its own device
+    if (e == cudaSuccess) e = c->arena.release();
+    if (e == cudaSuccess) e = cudaMemPoolTrimTo(c->pool, 0);
+    cudaSetDevice(cur);
   }
+  if (e != cudaSuccess) return fail(PA_ERR_CUDA, std::string("giving back memory: ") + cudaGetErrorString(e));
   return PA_OK;
 }
 
